@@ -482,6 +482,16 @@ __global__ void k_vertex(const PFSegment *__restrict__ segs, int nSegs, const PF
 // setup + binning
 // ---------------------------------------------------------------------------
 
+// Warp-wide exclusive prefix sum of v; total gets the sum over the warp.
+__device__ __forceinline__ uint32_t warp_offsets(uint32_t v, uint32_t &total)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t s = v;
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, s, o); if (lane >= o) s += t; }
+    total = __shfl_sync(0xffffffffu, s, 31);
+    return s - v;
+}
+
 struct BinArgs {
     uint32_t *binCount;
     uint32_t *tileList;        // the raster work lists
@@ -594,9 +604,10 @@ __device__ __forceinline__ void bin_slot(const BinArgs &B, uint32_t t, uint32_t 
 // longest tiles do not start last.
 __device__ __forceinline__ uint32_t heavy_level(uint32_t count)
 {
-    uint32_t l = 0;
-    for (uint32_t th = PF_HEAVY_BASE; l < PF_HEAVY_LEVELS && count >= th; th <<= 2) l++;
-    return l;                                          // 0: below the first level
+    uint32_t l = 0;                                    // 0: below the first level
+#pragma unroll
+    for (int k = 0; k < PF_HEAVY_LEVELS; k++) l += count >= ((uint32_t)PF_HEAVY_BASE << (2 * k)) ? 1u : 0u;
+    return l;
 }
 
 __device__ __forceinline__ void list_tile(const BinArgs &B, uint32_t t, uint32_t before, uint32_t added)
@@ -604,6 +615,28 @@ __device__ __forceinline__ void list_tile(const BinArgs &B, uint32_t t, uint32_t
     if (before == 0) B.tileList[atomicAdd(&B.cnt->tileListCount, 1u)] = t;
     for (uint32_t l = heavy_level(before) + 1; l <= heavy_level(before + added); l++)
         B.tileList[l * B.listStride + atomicAdd(&B.cnt->heavyCount[l - 1], 1u)] = t;
+}
+
+// The same for the tiles of a whole warp (every lane calls it; lanes that
+// put nothing on a list pass added = 0): one atomic a list and warp.  The
+// five counters share a cache line, so an atomic per tile and level queues
+// there: the batch of 64 soups, 83,000 tiles past most levels, k_items 777
+// -> 645 us.
+__device__ __forceinline__ void list_tiles_warp(const BinArgs &B, uint32_t t, uint32_t before, uint32_t added)
+{
+    const uint32_t from = heavy_level(before), to = heavy_level(before + added);
+    if (!__any_sync(0xffffffffu, added && (before == 0 || to > from))) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t l = 0; l <= PF_HEAVY_LEVELS; l++) {
+        const bool put = added && (l == 0 ? before == 0 : (from < l && l <= to));
+        const uint32_t m = __ballot_sync(0xffffffffu, put);
+        if (!m) continue;
+        const uint32_t first = (uint32_t)(__ffs(m) - 1);
+        uint32_t at = 0;
+        if (lane == first) at = atomicAdd(l == 0 ? &B.cnt->tileListCount : &B.cnt->heavyCount[l - 1], (unsigned)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, first);
+        if (put) B.tileList[l * B.listStride + at + __popc(m & ((1u << lane) - 1u))] = t;
+    }
 }
 
 // Append `key` to the bin of every tile the sub-triangle touches (one
@@ -623,90 +656,146 @@ __device__ void bin_prim(const BinArgs &B, const TileSpace &T, const PFPrim &P, 
         }
 }
 
-// Warp-cooperative binning: lanes whose sub-triangles touch the same tile
-// share one atomic on its counter (neighbouring triangles of a mesh usually
-// do); slots within a group follow lane order.  The counters of up to
-// BIN_BURST tiles are claimed before any of their slots is written, so that
-// the atomics' round trips overlap.  A sub-triangle touching more than
-// BIN_WIDE tiles is binned by the whole warp, 32 of its tiles at a time.
+// A lane's sub-triangle as its warp bins it, in shared memory: seven 16-byte
+// words (a stride of 28 banks: 16-byte reads of eight different records
+// touch every bank once).
+struct __align__(16) BinRec {
+    int32_t ex[3], ey[3], c[3];        // edge functions x ex + y ey + c (on), as EdgeTest
+    float rex[3];                      // 1 / ex
+    int32_t x0, x1, y0, y1;            // its pixels, inside the framebuffer (inclusive)
+    uint32_t on;
+    uint32_t first;                    // number of its first tile row
+    uint32_t tileBase, tilesX, key;
+    uint32_t pad[7];
+};
+static_assert(sizeof(BinRec) == 112, "seven 16-byte words");
+
+// A tile row of a sub-triangle: a run of tiles.
+struct __align__(16) BinRow {
+    uint32_t tile, first, key, pad;    // first tile, number of its first (row, tile) pair
+};
+
+// Binning scratch of a warp.
+struct BinWarp {
+    BinRec rec[32];
+    BinRow row[32];
+};
+
+// The pixel columns [lo, hi] of tile row ty that may hold covered pixels:
+// those where no edge function is negative on the whole of the row's part
+// of the column (the largest value is at one end of it), bounded by the
+// root of that value, which is linear in x.  The root is found in single
+// precision and widened by 1/32 of a pixel: |x| is below 2^13 and the
+// value's integer terms below 2^30, so its error stays below 2^-7; a column
+// too many costs nothing but a bin entry that covers no pixel.
+__device__ __forceinline__ void row_columns(const BinRec &r, uint32_t ty, int32_t &lo, int32_t &hi)
+{
+    lo = r.x0; hi = r.x1;
+    if (!r.on) return;
+    const int32_t y0 = max(r.y0, (int32_t)(ty * PF_TILE)), y1 = min(r.y1, (int32_t)(ty * PF_TILE + PF_TILE - 1));
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        const int32_t v = r.c[e] + r.ey[e] * (r.ey[e] > 0 ? y1 : y0);      // its largest over the row at x = 0
+        const float root = -(float)v * r.rex[e];
+        if (r.ex[e] > 0) lo = max(lo, __float2int_ru(root - 0.03125f));
+        else if (r.ex[e] < 0) hi = min(hi, __float2int_rd(root + 0.03125f));
+        else if (v < 0) hi = lo - 1;
+    }
+}
+
+// Warp-cooperative binning of the lanes' sub-triangles: the tile rows of all
+// of them are numbered through and each lane takes one, finding the run of
+// tiles the sub-triangle may cover there; then the (row, tile) pairs of 32
+// rows are numbered through and each lane takes one pair at a time.  So the
+// work is even whatever the sub-triangles' sizes, and only tiles that get
+// an entry are visited.  Bound by instruction issue and, in small launches,
+// by the round trips of the counter atomics.  Testing every tile of the box
+// instead, one sub-triangle after the other, a batch of 64 soups (207,000
+// items covering hundreds of tiles each, 4.5 tiles tested per entry) took
+// 614 us, now 305; phong1080, whose triangles cover one or two tiles, 285
+// -> 217 us; the 2,000-triangle soup at 256x256 136 -> 17 us together with
+// the items a warp (pfd_launch_items).  Pairs of one window of
+// 32 that touch the same tile share one atomic on its counter (neighbouring
+// triangles of a mesh usually do), slots within a group follow lane order;
+// the pairs of a single sub-triangle are distinct tiles and skip the
+// grouping.  The counters of BIN_BURST windows are claimed before any of
+// their slots is written, so that the atomics' round trips overlap.
 // Every lane of the warp must call it (lanes with nothing to bin pass
 // has = false).
 #define BIN_BURST 4
-#define BIN_WIDE 32
-__device__ void bin_prim_warp(const BinArgs &B, const TileSpace &T, bool has, const PFPrim &P, uint32_t key)
+__device__ void bin_prim_warp(const BinArgs &B, const TileSpace &T, bool has, const PFPrim &P, uint32_t key, BinWarp &S)
 {
+    const uint32_t all = 0xffffffffu;
     uint32_t tx0 = 0, ty0 = 0, ntx = 1, nty = 0;
-    if (has && !tile_range(T, P, tx0, ty0, ntx, nty)) has = false;
-    uint32_t n = has ? ntx * nty : 0;
+    if (has && !tile_range(T, P, tx0, ty0, ntx, nty)) nty = 0;
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1;
-    // large sub-triangles, one after the other: each lane takes tiles of it,
-    // each with its own counter (independent atomics)
-    for (uint32_t wide = __ballot_sync(0xffffffffu, n > BIN_WIDE); wide; wide &= wide - 1) {
-        const int src = __ffs(wide) - 1;
-        const uint32_t wx0 = __shfl_sync(0xffffffffu, tx0, src), wy0 = __shfl_sync(0xffffffffu, ty0, src);
-        const uint32_t wnx = __shfl_sync(0xffffffffu, ntx, src), wn = __shfl_sync(0xffffffffu, n, src);
-        const uint32_t wkey = __shfl_sync(0xffffffffu, key, src);
-        // the tile space of that lane's framebuffer (the lanes of a batch's
-        // warp may draw into different ones)
-        const uint32_t wbase = __shfl_sync(0xffffffffu, T.tileBase, src), wtx = __shfl_sync(0xffffffffu, T.tilesX, src);
-        const uint32_t wW = __shfl_sync(0xffffffffu, T.W, src), wH = __shfl_sync(0xffffffffu, T.H, src);
-        EdgeTest wb;
-        {
-            const EdgeTest mine = edge_test(P, T.W, T.H);
-            for (int e = 0; e < 3; e++) {
-                wb.ex[e] = __shfl_sync(0xffffffffu, mine.ex[e], src);
-                wb.ey[e] = __shfl_sync(0xffffffffu, mine.ey[e], src);
-                wb.c[e] = __shfl_sync(0xffffffffu, mine.c[e], src);
-            }
-            wb.xMin = __shfl_sync(0xffffffffu, mine.xMin, src); wb.xMax = __shfl_sync(0xffffffffu, mine.xMax, src);
-            wb.yMin = __shfl_sync(0xffffffffu, mine.yMin, src); wb.yMax = __shfl_sync(0xffffffffu, mine.yMax, src);
-            wb.on = __shfl_sync(0xffffffffu, (int)mine.on, src) != 0;
-        }
-        for (uint32_t i0 = 0; i0 < wn; i0 += 32u * BIN_BURST) {
-            uint32_t tt[BIN_BURST], bb[BIN_BURST];
-#pragma unroll
-            for (int u = 0; u < BIN_BURST; u++) {
-                const uint32_t i = i0 + 32u * (uint32_t)u + lane;
-                const bool hit = i < wn && tile_touched(wb, wx0 + i % wnx, wy0 + i / wnx, wW, wH);
-                tt[u] = hit ? wbase + (wy0 + i / wnx) * wtx + (wx0 + i % wnx) : 0xffffffffu;
-                bb[u] = hit ? atomicAdd(&B.binCount[tt[u]], 1u) : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < BIN_BURST; u++) {
-                if (tt[u] == 0xffffffffu) continue;
-                list_tile(B, tt[u], bb[u], 1u);
-                bin_slot(B, tt[u], bb[u], wkey);
-            }
-        }
+    const uint32_t lt = (1u << lane) - 1, le = lt | (1u << lane);
+    uint32_t rows;
+    const uint32_t firstRow = warp_offsets(nty, rows);
+    const uint32_t owners = __ballot_sync(all, nty > 0);
+    if (nty > 0) {
+        const EdgeTest E = edge_test(P, T.W, T.H);
+        BinRec r;
+        for (int e = 0; e < 3; e++) { r.ex[e] = E.ex[e]; r.ey[e] = E.ey[e]; r.c[e] = E.c[e]; r.rex[e] = __frcp_rn((float)E.ex[e]); }
+        r.x0 = P.xMin; r.x1 = (int32_t)min((uint32_t)P.xMax, T.W) - 1;
+        r.y0 = P.yMin; r.y1 = (int32_t)min((uint32_t)P.yMax, T.H - 1u);
+        r.on = E.on; r.first = firstRow;
+        r.tileBase = T.tileBase; r.tilesX = T.tilesX; r.key = key;
+        S.rec[__popc(owners & lt)] = r;
     }
-    if (n > BIN_WIDE) n = 0;
-    const EdgeTest ET = edge_test(P, T.W, T.H);
-    uint32_t most = n;
-    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-    for (uint32_t i0 = 0; i0 < most; i0 += BIN_BURST) {
-        uint32_t tt[BIN_BURST], gg[BIN_BURST], bb[BIN_BURST];
-#pragma unroll
-        for (int u = 0; u < BIN_BURST; u++) {
-            const uint32_t i = i0 + (uint32_t)u;
-            tt[u] = 0xffffffffu; gg[u] = 0; bb[u] = 0;
-            if (i >= most) continue;                           // uniform over the warp
-            const bool act = i < n && tile_touched(ET, tx0 + i % ntx, ty0 + i / ntx, T.W, T.H);
-            const uint32_t t = act ? T.tileBase + (ty0 + i / ntx) * T.tilesX + (tx0 + i % ntx) : 0xffffffffu;
-            const uint32_t grp = __match_any_sync(0xffffffffu, t);
-            tt[u] = t; gg[u] = grp;
-            if (act && lane == (uint32_t)(__ffs(grp) - 1)) bb[u] = atomicAdd(&B.binCount[t], (unsigned)__popc(grp));
+    __syncwarp();
+    for (uint32_t r0 = 0; r0 < rows; r0 += 32u) {
+        // my row: of the last sub-triangle whose first row is not past it
+        BinRow w{ 0, 0, 0, 0 };
+        uint32_t n = 0;
+        {
+            const uint32_t before = __popc(__ballot_sync(all, nty > 0 && firstRow < r0));
+            const uint32_t heads = __reduce_or_sync(all, (nty > 0 && firstRow - r0 < 32u) ? 1u << (firstRow - r0) : 0u);
+            if (r0 + lane < rows) {
+                const BinRec &r = S.rec[before + __popc(heads & le) - 1u];
+                const uint32_t ty = (uint32_t)r.y0 / PF_TILE + (r0 + lane - r.first);
+                int32_t lo, hi;
+                row_columns(r, ty, lo, hi);
+                if (lo <= hi) {
+                    n = (uint32_t)hi / PF_TILE - (uint32_t)lo / PF_TILE + 1u;
+                    w.tile = r.tileBase + ty * r.tilesX + (uint32_t)lo / PF_TILE;
+                }
+                w.key = r.key;
+            }
         }
+        uint32_t total;
+        w.first = warp_offsets(n, total);
+        const uint32_t filled = __ballot_sync(all, n > 0);
+        if (n > 0) S.row[__popc(filled & lt)] = w;
+        __syncwarp();
+        for (uint32_t p0 = 0; p0 < total; p0 += 32u * BIN_BURST) {
+            uint32_t tt[BIN_BURST], gg[BIN_BURST], bb[BIN_BURST], kk[BIN_BURST];
 #pragma unroll
-        for (int u = 0; u < BIN_BURST; u++) {
-            const uint32_t i = i0 + (uint32_t)u;
-            if (i >= most) continue;
-            const uint32_t grp = gg[u], leader = (uint32_t)(__ffs(grp) - 1);
-            const uint32_t base = __shfl_sync(0xffffffffu, bb[u], leader);
-            if (tt[u] == 0xffffffffu) continue;
-            if (lane == leader) list_tile(B, tt[u], base, (uint32_t)__popc(grp));
-            bin_slot(B, tt[u], base + __popc(grp & lt), key);
+            for (int u = 0; u < BIN_BURST; u++) {
+                const uint32_t w0 = p0 + 32u * (uint32_t)u, p = w0 + lane;
+                tt[u] = 0xffffffffu; gg[u] = 0; bb[u] = 0; kk[u] = 0;
+                if (w0 >= total) continue;                     // uniform over the warp
+                const uint32_t before = __popc(__ballot_sync(all, n > 0 && w.first < w0));
+                const uint32_t heads = __reduce_or_sync(all, (n > 0 && w.first - w0 < 32u) ? 1u << (w.first - w0) : 0u);
+                const BinRow q = S.row[before + __popc(heads & le) - 1u];    // (past the last pair: the last row)
+                const bool act = p < total;
+                const uint32_t t = act ? q.tile + (p - q.first) : 0xffffffffu;
+                const uint32_t key0 = __shfl_sync(all, q.key, 0);
+                const uint32_t grp = __all_sync(all, q.key == key0) ? 1u << lane : __match_any_sync(all, t);
+                tt[u] = t; gg[u] = grp; kk[u] = q.key;
+                if (act && lane == (uint32_t)(__ffs(grp) - 1)) bb[u] = atomicAdd(&B.binCount[t], (unsigned)__popc(grp));
+            }
+#pragma unroll
+            for (int u = 0; u < BIN_BURST; u++) {
+                if (p0 + 32u * (uint32_t)u >= total) continue;
+                const uint32_t grp = gg[u], leader = (uint32_t)(__ffs(grp) - 1);
+                const uint32_t base = __shfl_sync(all, bb[u], leader);
+                const bool act = tt[u] != 0xffffffffu;
+                list_tiles_warp(B, tt[u], base, act && lane == leader ? (uint32_t)__popc(grp) : 0u);
+                if (act) bin_slot(B, tt[u], base + __popc(grp & lt), kk[u]);
+            }
         }
+        __syncwarp();                                          // the rows are free
     }
 }
 
@@ -973,20 +1062,23 @@ __device__ __forceinline__ bool item_setup(const PFSegment &sg, const PFDrawStat
     return true;
 }
 __global__ void __launch_bounds__(128, 6) k_items(const PFSegment *__restrict__ segs, int nSegs, const PFDrawState *__restrict__ states,
-                        const PFVertexOut *__restrict__ vout, uint32_t nItems, ItemOut O, BinArgs B)
+                        const PFVertexOut *__restrict__ vout, uint32_t nItems, uint32_t perWarp, ItemOut O, BinArgs B)
 {
     __shared__ int sUniform, sAborted;
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ BinWarp sBin[4];
+    // a warp's first perWarp lanes set up an item each, all of its lanes bin
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t g0 = blockIdx.x * 4u * perWarp;
+    const uint32_t g = lane < perWarp ? g0 + warp * perWarp + lane : 0xffffffffu;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // k_vertex is done
     // Thread 0 takes the block's decisions, behind one barrier: whether an
     // overflow in this launch has flagged the abort (other blocks set it
     // while this one runs; a thread that returned alone would leave the rest
     // of the block with unset shared state), and the segment of the block's
     // items when they share one (the usual case; the others search).
-    const uint32_t g0 = blockIdx.x * blockDim.x;
     if (threadIdx.x == 0) {
         sAborted = B.cnt->abortCommand != 0xffffffffu;
-        const int a = seg_of_item(segs, nSegs, g0), b = seg_of_item(segs, nSegs, min(g0 + blockDim.x, nItems) - 1);
+        const int a = seg_of_item(segs, nSegs, g0), b = seg_of_item(segs, nSegs, min(g0 + 4u * perWarp, nItems) - 1);
         sUniform = (a == b) ? a : -1;
     }
     __syncthreads();
@@ -1007,11 +1099,11 @@ __global__ void __launch_bounds__(128, 6) k_items(const PFSegment *__restrict__ 
     // round trip, no block barrier)
     const unsigned wk = __popc(__ballot_sync(0xffffffffu, kept));
     if ((threadIdx.x & 31) == 0 && wk) atomicAdd(&B.cnt->batchRasterized, (unsigned long long)wk);
-    if (O.rowInfo) {                                   // the warp's summary for k_rows
+    if (O.rowInfo) {                                   // the warp's summary for k_rows (perWarp is 32)
         const uint64_t grp = row_group(g < nItems ? O.rowInfo[g] : 0ull);
         if ((threadIdx.x & 31) == 0) O.rowGroup[g >> 5] = grp;
     }
-    bin_prim_warp(B, T, kept, P, g << PF_SUB_BITS);
+    bin_prim_warp(B, T, kept, P, g << PF_SUB_BITS, sBin[warp]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1463,16 +1555,6 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x)
         x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
     }
     return x;
-}
-
-// Warp-wide exclusive prefix sum of v; total gets the sum over the warp.
-__device__ __forceinline__ uint32_t warp_offsets(uint32_t v, uint32_t &total)
-{
-    const int lane = threadIdx.x & 31;
-    uint32_t s = v;
-    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, s, o); if (lane >= o) s += t; }
-    total = __shfl_sync(0xffffffffu, s, 31);
-    return s - v;
 }
 
 template <bool GEN, int WARPS>
@@ -2167,8 +2249,18 @@ cudaError_t pfd_launch_items(const PFBatchLaunch &L, cudaStream_t st)
     if (L.nItems == 0) return cudaSuccess;
     BinArgs B{ L.binCount, L.tileList, L.listStride, L.bins, L.cap, L.targets, L.cnt, L.command };
     ItemOut O{ L.prims, L.primsPh, L.pool, L.poolPh, L.poolCap, L.rowCount ? L.rowInfo : nullptr, L.rowGroup };
-    return launch_serialized(k_items, grid_for(L.nItems, 128), 128, 0, st, L.segs, L.nSegs, L.states,
-                             (const PFVertexOut *)L.vout, L.nItems, O, B);
+    // Items a warp: a full warp of 32 sets up fastest, but a small launch
+    // then leaves most of the GPU idle while a few warps bin all its tiles.
+    // Fewer items a warp until there are 12 warps an SM (half of what is
+    // resident; all 24 measured slower): 2,000 soup triangles 66 (32 a warp)
+    // -> 16 us (1), 8,192 small ones 20 -> 12 us (4; 2: 15.5), 20,480 mesh
+    // items 22.5 -> 12.5 us (8; 4: 15); 131,072 stay at 32 (20.6 us; 16: 22).
+    // k_rows' summaries are one a warp of 32.
+    uint32_t perWarp = 32;
+    if (!O.rowInfo)
+        while (perWarp > 1 && L.nItems / perWarp < (uint32_t)pfd_sm_count() * 12u) perWarp >>= 1;
+    return launch_serialized(k_items, grid_for(L.nItems, 4 * perWarp), 128, 0, st, L.segs, L.nSegs, L.states,
+                             (const PFVertexOut *)L.vout, L.nItems, perWarp, O, B);
 }
 
 // Dynamic shared memory of k_raster: the warps' batch buffers (a record's
