@@ -1121,11 +1121,13 @@ __global__ void __launch_bounds__(128, 6) k_items(const PFSegment *__restrict__ 
 //   1. every lane loads one record of the batch into the warp's shared
 //      memory and derives its edge functions at the tile origin and its
 //      bounding box clipped to the tile;
-//   2. each lane walks the batch in order at its own two pixels: coverage
-//      with the reference's integer edge functions, depth, depth test and
-//      depth write (triangles.c:398-438) -- which leaves, per pixel, the
-//      fragments that passed (bit k of a 32-bit mask: the record's place in
-//      the batch);
+//   2. from the second batch on, records that lie behind every pixel of the
+//      tile are dropped (their covered pixels still count); each lane walks
+//      the others in order at its own two pixels: coverage with the
+//      reference's integer edge functions, depth, depth test and depth write
+//      (triangles.c:398-438) -- which leaves, per pixel, the fragments that
+//      passed and are not replaced by a later unblended one (bit k of a
+//      32-bit mask: the record's place in the batch);
 //   3. the passing fragments are listed pixel by pixel in submission order
 //      and shaded densely over the warp (texture, Gouraud / Phong colour:
 //      the source colour does not depend on the destination);
@@ -1193,6 +1195,7 @@ struct QWarp {
     SPrim rec[QCHN];
     QEdge edge[QCHN];
     uint32_t keys[REG_SORT_MAX];   // a short bin's keys in submission order (sorted in registers)
+    uint32_t pend[PF_TILE_PIXELS]; // per pixel (32 slot + lane) the bin key of its fragment that waits to be shaded
     uint16_t fdesc[QFW];       // listed fragments: tile pixel << 5 | record
     uint32_t fc[QFW];          // their colour
 };
@@ -1231,6 +1234,62 @@ __device__ __forceinline__ void tile_edge(const int4 q0, const int4 q1, const in
     E.zReject = zReject;
 }
 
+// Order-preserving integer key of a depth: keys compare as the depths do,
+// NaN above everything.
+__device__ __forceinline__ uint32_t depth_key(float d)
+{
+    const uint32_t u = (uint32_t)__float_as_int(d);
+    return d != d ? 0xffffffffu : u ^ ((int32_t)u < 0 ? 0xffffffffu : 0x80000000u);
+}
+
+// A tile's depth-test rejection bound of a record whose box reaches past
+// the tile (depth_reject_bound, over the tile's part of the box instead of
+// the whole triangle).  The interpolated term zs is affine in the pixel, so
+// over the box it is at most its value at one corner plus the steps to the
+// largest one; m bounds the sum of the absolute terms, and 2e-6 m the
+// rounding of this evaluation (a dozen operations of 2^-24 each) and of a
+// covered fragment's own terms (their sum there is at most m).  The
+// corners' depths of a wide triangle say little about its depth in one tile:
+// with this bound most records behind the tile's pixels are dropped whole
+// (k_raster: 64-soup batch 3,017 -> 1,925 us, soup256 139 -> 65 us).  zq:
+// wInvSum, z1, z2, z3.
+__device__ __forceinline__ float tile_reject(const QEdge &E, const float4 zq)
+{
+    const float bound = E.zReject;
+    if (!(bound == bound)) return bound;                     // no bound: func, depth test or signs
+    const uint32_t bx0 = E.box & 15u, bw = (E.box >> 4) & 15u, by0 = (E.box >> 8) & 15u, bh = (E.box >> 12) & 15u;
+    const float dx = (float)bw - 1.0f, dy = (float)bh - 1.0f;
+    const int32_t ex[3] = { E.ex0, E.ex1, E.ex2 }, ey[3] = { E.ey0, E.ey1, E.ey2 };
+    const float z[3] = { zq.y, zq.z, zq.w };
+    float a = 0.0f, gx = 0.0f, gy = 0.0f, m = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        const int32_t w = (int32_t)((uint32_t)E.e0[e] + bx0 * (uint32_t)ex[e] + by0 * (uint32_t)ey[e]);
+        const float zw = z[e] * zq.x, fw = (float)w, fx = (float)ex[e], fy = (float)ey[e];
+        a += fw * zw; gx += fx * zw; gy += fy * zw;
+        m += (fabsf(fw) + fabsf(fx) * dx + fabsf(fy) * dy) * fabsf(zw);
+    }
+    const float top = a + fmaxf(gx * dx, 0.0f) + fmaxf(gy * dy, 0.0f) + 2e-6f * m;
+    const float lo = fminf(z[0], fminf(z[1], z[2])), hi = fminf(top, fmaxf(z[0], fmaxf(z[1], z[2])));
+    float b;
+    if (lo > 0.0f) {
+        if (!(hi > 0.0f)) return bound;
+        b = __frcp_rn(hi * 1.00001f) * 0.9999899f;
+    } else {
+        if (!(hi < 0.0f)) return bound;
+        b = __frcp_rn(hi * 0.99999f) * 1.0000101f;
+    }
+    return fabsf(b) < 1e30f ? fmaxf(b, bound) : bound;
+}
+
+// Whether the record may raise a pixel's depth (a batch without such
+// records only lowers depths).
+__device__ __forceinline__ bool raises_depth(uint32_t rstate)
+{
+    const uint32_t func = (rstate >> 16) & 255u;
+    return (rstate & PFS_DEPTH_MASK) && !((rstate & PFS_DEPTH_TEST) && (func == 2u || func == 3u || func == 0u));
+}
+
 // Normalised weights and depth of a covered fragment at tile pixel (X, Y)
 // (triangles.c:421-438).
 __device__ __forceinline__ float tile_depth(const QEdge &E, const PFPrim &P, uint32_t X, uint32_t Y, float *wn)
@@ -1250,6 +1309,7 @@ __device__ __forceinline__ float tile_depth(const QEdge &E, const PFPrim &P, uin
 // reference replaces by zero before sampling (triangles.c:508-513);
 // anyWeights: the pixel may lie outside the triangle (weights outside
 // [0, 1]), so the weight conversions follow CVTPS2DQ out of range too.
+template <bool PHONG>
 __device__ __forceinline__ uint32_t shade_fragment(const PFPrim &P, const PFPrimPhong *Q, const PFDrawState *states,
                                                    float wn1, float wn2, float wn3, float z,
                                                    bool texOn = true, bool anyWeights = false)
@@ -1284,7 +1344,7 @@ __device__ __forceinline__ uint32_t shade_fragment(const PFPrim &P, const PFPrim
         }
         frag = blend_simd(4, tex_sample(tex_desc(P, states), tu, tv), frag);
     }
-    if (fl & PFS_PHONG) {
+    if (PHONG && (fl & PFS_PHONG)) {
         const PFDrawState &S = states[P.flags >> 8];
         PFPrimPhong q;                                  // (80 bytes, five 16-byte loads)
         for (int i = 0; i < 5; i++) reinterpret_cast<float4 *>(&q)[i] = __ldg(reinterpret_cast<const float4 *>(Q) + i);
@@ -1557,7 +1617,12 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x)
     return x;
 }
 
-template <bool GEN, int WARPS>
+// GEN: a target is not RGBA / unsigned byte.  PHONG: a draw state lights per
+// fragment; without that code the 80 registers hold everything (with it 52
+// bytes a thread spill): sphere1080 58 -> 56 us, 64-soup batch 1,925 ->
+// 1,780.  Bound by instruction issue and the round trips of claims, bin keys
+// and records.
+template <bool GEN, int WARPS, bool PHONG>
 __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
 {
     extern __shared__ __align__(16) unsigned char rsmem[];
@@ -1569,7 +1634,7 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
     // the batch completed set-up without overflow: its sub-triangles count
     if (blockIdx.x == 0 && tid == 0) atomicAdd(&a.cnt->rasterized, a.cnt->batchRasterized);
     const uint32_t lx = (uint32_t)lane & 7u, ly = (uint32_t)lane >> 3;     // my pixels: (lx, ly) and (lx, ly + 4)
-    unsigned long long frags = 0;
+    uint32_t frags = 0;                                // (at most 64 a bin entry and tile)
 
     // persistent: warps take tiles from a shared work queue -- the tiles the
     // binning listed as non-empty, those of the heaviest level first, then
@@ -1577,42 +1642,47 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
     // first list it is on and skipped on the later ones); then the groups of
     // 32 tiles whose empty bins only get their fused clear, if any, one tile
     // a lane
-    uint32_t levelEnd[PF_HEAVY_LEVELS + 1];           // queue index past level l's entries, heaviest first
-    uint32_t nQueue = 0;
     // A heavy level with few tiles against the grid's warps sets the end of
     // the launch (its tiles start first but run longest): each of its tiles
     // is then two work items, its top and bottom halves, each a warp with
     // one pixel a lane, which take about half as long.  Where heavy tiles
     // are many the launch is bound by the total work, which halves would
     // only add to (each half walks the whole bin).
-    uint32_t splitLevels = 0;
-    for (int l = PF_HEAVY_LEVELS; l >= 1; l--) {
-        const uint32_t c = min(a.cnt->heavyCount[l - 1], a.totalTiles);
-        const bool split = 4u * c <= gridDim.x * (uint32_t)WARPS;
-        splitLevels |= split ? 1u << l : 0u;
-        nQueue += split ? 2u * c : c;
-        levelEnd[l] = nQueue;
+    // (in shared memory, like the fragment count: read by lane 0 between
+    // tiles only, they would cost the tile's loops registers)
+    __shared__ uint32_t sLevelEnd[PF_HEAVY_LEVELS + 1];    // queue index past level l's entries, heaviest first
+    __shared__ uint32_t sSplit;
+    __shared__ unsigned long long sFrags;
+    if (tid == 0) {
+        uint32_t nQueue = 0, split = 0;
+        for (int l = PF_HEAVY_LEVELS; l >= 1; l--) {
+            const uint32_t c = min(a.cnt->heavyCount[l - 1], a.totalTiles);
+            const bool sp = 4u * c <= gridDim.x * (uint32_t)WARPS;
+            split |= sp ? 1u << l : 0u;
+            nQueue += sp ? 2u * c : c;
+            sLevelEnd[l] = nQueue;
+        }
+        sLevelEnd[0] = nQueue + min(a.cnt->tileListCount, a.totalTiles);
+        sSplit = split;
+        sFrags = 0;
     }
-    nQueue += min(a.cnt->tileListCount, a.totalTiles);
-    levelEnd[0] = nQueue;
-    const uint32_t nClear = (a.totalTiles + 31u) / 32u;
+    __syncthreads();
     // each warp's first entry is its own index in the grid; the counter
     // hands out the entries after those (3,648 warps claiming their first
     // entry with one atomic each would serialise at the start)
-    const uint32_t gridWarps = gridDim.x * (uint32_t)WARPS;
     uint32_t claim = blockIdx.x * (uint32_t)WARPS + (uint32_t)warp;
     for (;;) {
     uint32_t next = 0xffffffffu, nextCount = 0;
     if (lane == 0) {
-        const uint32_t q = claim;
-        if (q < nQueue + nClear) {
-            claim = gridWarps + atomicAdd(&a.cnt->tileQueue, 1u);
+        const uint32_t q = claim, nQueue = sLevelEnd[0];
+        if (q < nQueue + (a.totalTiles + 31u) / 32u) {
+            claim = gridDim.x * (uint32_t)WARPS + atomicAdd(&a.cnt->tileQueue, 1u);
             if (q >= nQueue) next = 0x80000000u | (q - nQueue);      // a group of tiles to clear
             else {
                 uint32_t level = PF_HEAVY_LEVELS, begin = 0;
-                while (q >= levelEnd[level]) { begin = levelEnd[level]; level--; }
+                while (q >= sLevelEnd[level]) { begin = sLevelEnd[level]; level--; }
                 const uint32_t e = q - begin;
-                const bool split = (splitLevels >> level) & 1u;
+                const bool split = (sSplit >> level) & 1u;
                 next = __ldg(a.tileList + (size_t)level * a.listStride + (split ? e >> 1 : e));
                 nextCount = __ldg(a.binCount + next);
                 if (heavy_level(nextCount) != level) next = 0xfffffffeu;   // rasterized from an earlier list
@@ -1740,34 +1810,78 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
         __syncwarp();
     }
 
-    for (uint32_t c0 = 0; c0 < n; c0 += QCHN) {
-        const uint32_t cn = min((uint32_t)QCHN, n - c0);
+    // Where fragments are lit one by one (PHONG), unblended ones wait: in a
+    // tile of several batches, a pixel's fragment that nothing of its batch
+    // blends over is kept as its bin key (Q.pend) and shaded only when a
+    // batch with blended records comes, or at the end -- most are replaced
+    // before that (phong1080: about three of a pixel's fragments pass, one
+    // is seen; k_raster 520 -> 405 us).  Without per-fragment lighting the
+    // bookkeeping costs more than it saves (64-soup batch 1,925 -> 2,255 us,
+    // sphere1080 58 -> 65).  Shading those that wait is a
+    // batch of its own per pixel slot (phase 1 and 2), whose records are the
+    // lanes' own; it ends the waiting, so that draws that alternate between
+    // blended and unblended records pay for it once a tile.
+    bool defer = n > QCHN, pending = false;
+    uint32_t ph = 0, c0 = 0;
+    for (;;) {
+        if (ph == 0 && c0 >= n) {
+            if (!PHONG || !pending) break;
+            ph = 1;
+        }
+        const uint32_t phase = PHONG ? ph : 0u;
+        // the farthest depth of the tile's pixels, from the second batch on
+        // (a tile of one batch has nothing in front yet)
+        const uint32_t farKey = c0 == 0 || phase != 0 ? 0xffffffffu :
+            __reduce_max_sync(0xffffffffu, max(in0 ? depth_key(dep0) : 0u, in1 ? depth_key(dep1) : 0u));
         // 1. my record: load, stage, derive its tile set-up and coverage
         uint32_t kind = 0;
         unsigned long long covMask = 0;
-        if ((uint32_t)lane < cn) {
-            uint32_t key;
-            if (!regSort) key = __ldg(bin + c0 + lane);
-            else key = Q.keys[c0 + (uint32_t)lane];
+        bool raises = false, hidden = false, blends = false;
+        uint32_t key = 0xffffffffu;
+        if (phase != 0) key = Q.pend[32u * (phase - 1u) + (uint32_t)lane];
+        else if (c0 + (uint32_t)lane < n) key = regSort ? Q.keys[c0 + (uint32_t)lane] : __ldg(bin + c0 + lane);
+        const bool have = key != 0xffffffffu;
+        if (have) {
             const uint32_t item = key >> PF_SUB_BITS, sub = key & ((1u << PF_SUB_BITS) - 1);
             const PFPrim *src = &a.prims[item];
             uint32_t pi = item;
             if (sub != 0) { pi = (uint32_t)__ldg(&a.prims[item].poolBase) + sub - 1; src = &a.pool[pi]; }
-            const int4 *s4 = reinterpret_cast<const int4 *>(src);
-            int4 r[8];
-            for (int i = 0; i < 8; i++) r[i] = __ldg(s4 + i);
-            int4 *d4 = reinterpret_cast<int4 *>(&Q.rec[lane].p);
-            for (int i = 0; i < 8; i++) d4[i] = r[i];
-            Q.rec[lane].ph = a.anyPhong ? (sub != 0 ? &a.poolPh[pi] : &a.primsPh[item]) : nullptr;
+            // (straight into shared memory: through registers, the record's 32
+            // words would spill what the tile holds)
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Q.rec[lane].p);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16u * i), "l"((const char *)src + 16 * i) : "memory");
+            if (PHONG) Q.rec[lane].ph = sub != 0 ? &a.poolPh[pi] : &a.primsPh[item];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            const int4 *r = reinterpret_cast<const int4 *>(&Q.rec[lane].p);
+            const int4 r1 = r[1], r2 = r[2];
             QEdge E;
-            tile_edge(r[0], r[1], r[2], (uint32_t)r[4].w, __int_as_float(r[6].z), ox, oy, W, H, E);
-            Q.edge[lane] = E;
-            kind = (uint32_t)r[2].z & PFP_KIND;
+            tile_edge(r[0], r1, r2, Q.rec[lane].p.rstate, Q.rec[lane].p.zReject, ox, oy, W, H, E);
+            kind = (uint32_t)r2.z & PFP_KIND;
+            raises = raises_depth(E.rstate);
+            blends = (E.rstate & PFS_BLEND) != 0;
             // my record's coverage of the tile, bit 8 y + x: the pixels of its
             // box that pass the integer edge test (triangles.c:398-424) or,
             // for a point, line or rectangle, its own rule
             const uint32_t bx0 = E.box & 15u, bw = (E.box >> 4) & 15u, by0 = (E.box >> 8) & 15u, bh = (E.box >> 12) & 15u;
-            if (kind == 0) {
+            if (phase != 0) {
+                // (covered and visible already)
+            } else if (kind == 0) {
+                // the whole box when no edge function is negative at its
+                // least corner (with these bounds none wraps inside the tile)
+                bool full = bw + bh >= 12u;
+                if (full)
+#pragma unroll
+                for (int e = 0; e < 3; e++) {
+                    const int32_t ex = e == 0 ? E.ex0 : e == 1 ? E.ex1 : E.ex2, ey = e == 0 ? E.ey0 : e == 1 ? E.ey1 : E.ey2;
+                    full = full && abs(E.e0[e]) < (1 << 30) && abs(ex) < (1 << 24) && abs(ey) < (1 << 24) &&
+                           E.e0[e] + (int32_t)(ex > 0 ? bx0 : bx0 + bw - 1u) * ex + (int32_t)(ey > 0 ? by0 : by0 + bh - 1u) * ey >= 0;
+                }
+                if (full) {
+                    covMask = (unsigned long long)(((1u << bw) - 1u) << bx0) * 0x0101010101010101ull;
+                    covMask &= (~0ull >> (64u - 8u * bh)) << (8u * by0);
+                } else
                 for (uint32_t y = by0; y < by0 + bh; y++) {
                     uint32_t w1 = (uint32_t)E.e0[0] + bx0 * (uint32_t)E.ex0 + y * (uint32_t)E.ey0;
                     uint32_t w2 = (uint32_t)E.e0[1] + bx0 * (uint32_t)E.ex1 + y * (uint32_t)E.ey1;
@@ -1779,14 +1893,35 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
                     }
                     covMask |= (unsigned long long)(row << bx0) << (8u * y);
                 }
+                if (n > QCHN && ((uint32_t)r2.x - (uint32_t)r1.z > bw || (uint32_t)r2.y - (uint32_t)r1.w >= bh))
+                    E.zReject = tile_reject(E, reinterpret_cast<const float4 *>(r)[3]);
+                hidden = E.zReject == E.zReject && depth_key(E.zReject) >= farKey;
             } else {
                 const PFPrim &P = Q.rec[lane].p;
                 for (uint32_t y = by0; y < by0 + bh; y++)
                     for (uint32_t x = bx0; x < bx0 + bw; x++)
                         if (lp_covers(P, (int32_t)(ox + x), (int32_t)(oy + y))) covMask |= 1ull << (8u * y + x);
             }
+            Q.edge[lane] = E;
         }
         const bool anyLP = __any_sync(0xffffffffu, kind != 0);
+        uint32_t vis0 = 0, vis1 = 0;                    // bit k: record k passed at my pixel of slot 0 / 1
+        if (phase != 0) {
+            if (phase == 1) vis0 = have ? 1u << lane : 0u; else vis1 = have ? 1u << lane : 0u;
+            __syncwarp();
+        } else {
+        // a record behind every pixel of the tile has no fragment that passes
+        // (no record of the batch raises a depth): its covered pixels count,
+        // and that is all
+        const bool lowers = __all_sync(0xffffffffu, !raises);
+        const bool live = covMask != 0 && !(lowers && hidden);
+        if (PHONG && pending && __any_sync(0xffffffffu, live && blends)) { ph = 1; __syncwarp(); continue; }
+        if (!live) {
+            // (a half tile: its own rows)
+            frags += (whole || rowA == ly ? __popc((uint32_t)covMask) : 0) + (whole || rowA != ly ? __popc((uint32_t)(covMask >> 32)) : 0);
+            covMask = 0;
+        }
+        if (!__any_sync(0xffffffffu, live)) { c0 += QCHN; continue; }
         __syncwarp();
         // 2a. coverage per pixel: bit k of cm0 / cm1 -- record k covers my
         //     pixel of slot 0 / 1 -- the records' masks transposed over the
@@ -1798,7 +1933,6 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
         // 2b. depth: each of my pixels walks its covering records in
         //     submission order -- depth (the correctly rounded reciprocal),
         //     the depth-test rejection bound, the depth test and write
-        uint32_t vis0 = 0, vis1 = 0;                    // bit k: record k passed at my pixel of slot 0 / 1
         uint32_t cov = 0;
         auto depth_walk = [&](uint32_t cm, float &d, uint32_t &vis, uint32_t row, uint32_t Y) {
             for (; cm; cm &= cm - 1) {
@@ -1830,13 +1964,33 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
                     z = lp_depth(P, (int32_t)X0, (int32_t)Y);
                     if ((rs & PFS_DEPTH_TEST) && !depth_sisd(func, z, d)) continue;
                 }
-                vis |= 1u << k;
+                // (an unblended fragment replaces what the batch drew here before:
+                // those fragments are never shaded)
+                vis = ((rs & PFS_BLEND) ? vis : 0u) | 1u << k;
                 if (rs & PFS_DEPTH_MASK) d = z;
             }
         };
         depth_walk(cm0, dep0, vis0, rowA, Y0);
         depth_walk(cm1, dep1, vis1, ly + 4u, Y1);
         frags += cov;
+        if (PHONG && defer) {
+            auto waits = [&](uint32_t vis) {
+                return vis && !(vis & (vis - 1u)) && !(Q.edge[__ffs(vis) - 1].rstate & PFS_BLEND);
+            };
+            const bool d0 = waits(vis0), d1 = waits(vis1);
+            if (__any_sync(0xffffffffu, d0 || d1)) {
+                auto key_of = [&](uint32_t vis) {
+                    const uint32_t i = c0 + (uint32_t)(__ffs(vis) - 1);
+                    return regSort ? Q.keys[i] : __ldg(bin + i);
+                };
+                if (d0 || !pending) Q.pend[lane] = d0 ? key_of(vis0) : 0xffffffffu;
+                if (d1 || !pending) Q.pend[32 + lane] = d1 ? key_of(vis1) : 0xffffffffu;
+                if (d0) vis0 = 0;
+                if (d1) vis1 = 0;
+                pending = true;
+            }
+        }
+        }
         // 3+4. shade the fragments that passed, densely over the warp, and
         //      blend each pixel's in submission order
         uint32_t totalv;
@@ -1856,7 +2010,7 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
                 }
                 float wn[3];
                 const float z = tile_depth(Q.edge[k], P, X, Y, wn);
-                Q.fc[f - b0] = shade_fragment(P, Q.rec[k].ph, a.states, wn[0], wn[1], wn[2], z);
+                Q.fc[f - b0] = shade_fragment<PHONG>(P, Q.rec[k].ph, a.states, wn[0], wn[1], wn[2], z);
             }
             __syncwarp();
             if (cntv && offv < bEnd && offv + cntv > b0) {
@@ -1880,17 +2034,25 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
             __syncwarp();                                  // the window's lists are free
         }
         __syncwarp();                                      // the batch's records are free
+        if (phase == 0) c0 += QCHN;
+        else if (phase == 1 && whole) ph = 2;
+        else { ph = 0; pending = false; defer = false; }
     }
-    if (in0) { col0.store(T, pidx0); T.depth[pidx0] = dep0; }
-    if (in1) { col1.store(T, pidx1); T.depth[pidx1] = dep1; }
+    {
+        // (indices from the target again: held through the batches they
+        // would cost registers)
+        const size_t p0 = (size_t)(oy + rowA) * T.W + ox + lx;
+        if (in0) { col0.store(T, p0); T.depth[p0] = dep0; }
+        const size_t p1 = (size_t)(oy + rowA + 4u) * T.W + ox + lx;
+        if (in1) { col1.store(T, p1); T.depth[p1] = dep1; }
+    }
+    if (frags >= 0x40000000u) { atomicAdd(&sFrags, (unsigned long long)frags); frags = 0; }
     }   // tile loop
 
     // fragment counter: one atomic per CTA (same-address atomics serialise)
-    __shared__ unsigned long long sFrags;
-    if (tid == 0) sFrags = 0;
-    __syncthreads();
-    for (int o = 16; o > 0; o >>= 1) frags += __shfl_down_sync(0xffffffffu, frags, o);
-    if (lane == 0 && frags) atomicAdd(&sFrags, frags);
+    unsigned long long all = frags;
+    for (int o = 16; o > 0; o >>= 1) all += __shfl_down_sync(0xffffffffu, all, o);
+    if (lane == 0 && all) atomicAdd(&sFrags, all);
     __syncthreads();
     if (tid == 0 && sFrags) atomicAdd(&a.cnt->fragments, sFrags);
 }
@@ -1966,7 +2128,7 @@ __device__ __noinline__ uint32_t row_record(const PFPrim &P, const PFPrimPhong *
             }
             if (!any) continue;
             // the half's value: its first pixel's colour and destination
-            uint32_t frag = shade_fragment(P, ph, states, wf[0], wf[1], wf[2], zf, m[0], true);
+            uint32_t frag = shade_fragment<true>(P, ph, states, wf[0], wf[1], wf[2], zf, m[0], true);
             if (rs & PFS_BLEND) frag = blend_simd(mode, frag, pff_swap_rb(crow[xf]));
             const uint32_t out = pff_swap_rb(frag);
             for (uint32_t j = 0; j < 4; j++) {
@@ -2302,14 +2464,19 @@ cudaError_t pfd_launch_binsort(const PFBatchLaunch &L, cudaStream_t st)
     return launch_serialized(k_binsort, grid, SORT_THREADS, smem, st, raster_args(L));
 }
 
+template <bool GEN, bool PHONG> static void (*raster_kernel(int warps))(RasterArgs)
+{
+    return warps == 2 ? k_raster<GEN, 2, PHONG> : warps == 8 ? k_raster<GEN, 8, PHONG> : k_raster<GEN, 4, PHONG>;
+}
+
 cudaError_t pfd_launch_raster(const PFBatchLaunch &L, cudaStream_t st)
 {
     if (L.totalTiles == 0) return cudaSuccess;
     const int warps = (L.rasterWarps == 2 || L.rasterWarps == 8) ? L.rasterWarps : 4;
     const size_t smem = raster_smem(warps);
     void (*kernel)(RasterArgs) =
-        L.generic ? (warps == 2 ? k_raster<true, 2> : warps == 8 ? k_raster<true, 8> : k_raster<true, 4>)
-                  : (warps == 2 ? k_raster<false, 2> : warps == 8 ? k_raster<false, 8> : k_raster<false, 4>);
+        L.generic ? (L.anyPhong ? raster_kernel<true, true>(warps) : raster_kernel<true, false>(warps))
+                  : (L.anyPhong ? raster_kernel<false, true>(warps) : raster_kernel<false, false>(warps));
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)     // the CTAs' shared memory, not L1, bounds how many fit on an SM
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
