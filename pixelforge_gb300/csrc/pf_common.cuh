@@ -176,3 +176,47 @@ __device__ bool setup_prim(const PFDrawState &S, int face, bool is3D, const SVer
     }
     return true;
 }
+
+// ---------------------------------------------------------------------------
+// warp helpers
+// ---------------------------------------------------------------------------
+// 32x32 bit matrix held one row a lane (bit j of lane k) -> one column a
+// lane: lane j gets bit k = bit j of lane k.  Five exchange steps, each
+// swapping the off-diagonal s x s blocks between lanes k and k ^ s.
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t masks[5] = { 0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u };
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        const uint32_t s = 16u >> i, m = masks[i];
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, (int)s);
+        x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
+    }
+    return x;
+}
+
+// Place of the set bit of m with k set bits below it (m has more than k).
+__device__ __forceinline__ uint32_t nth_bit(uint32_t m, uint32_t k)
+{
+    uint32_t at = 0;
+#pragma unroll
+    for (uint32_t s = 16; s > 0; s >>= 1) {
+        const uint32_t c = (uint32_t)__popc(m & ((1u << s) - 1u));
+        const bool up = k >= c;
+        k -= up ? c : 0u;
+        m = up ? m >> s : m;
+        at += up ? s : 0u;
+    }
+    return at;
+}
+
+// Warp-wide exclusive prefix sum of v; total gets the sum over the warp.
+__device__ __forceinline__ uint32_t warp_offsets(uint32_t v, uint32_t &total)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t s = v;
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, s, o); if (lane >= o) s += t; }
+    total = __shfl_sync(0xffffffffu, s, 31);
+    return s - v;
+}

@@ -482,16 +482,6 @@ __global__ void k_vertex(const PFSegment *__restrict__ segs, int nSegs, const PF
 // setup + binning
 // ---------------------------------------------------------------------------
 
-// Warp-wide exclusive prefix sum of v; total gets the sum over the warp.
-__device__ __forceinline__ uint32_t warp_offsets(uint32_t v, uint32_t &total)
-{
-    const int lane = threadIdx.x & 31;
-    uint32_t s = v;
-    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, s, o); if (lane >= o) s += t; }
-    total = __shfl_sync(0xffffffffu, s, 31);
-    return s - v;
-}
-
 struct BinArgs {
     uint32_t *binCount;
     uint32_t *tileList;        // the raster work lists
@@ -1599,22 +1589,6 @@ __device__ __forceinline__ void tile_list(unsigned long long m, uint32_t off, ui
         const uint32_t b = (uint32_t)(__ffsll(mm) - 1);
         fdesc[f - b0] = (uint16_t)(((lane + 32u * (b >> 5)) << 5) | (b & 31u));
     }
-}
-
-// 32x32 bit matrix held one row a lane (bit j of lane k) -> one column a
-// lane: lane j gets bit k = bit j of lane k.  Five exchange steps, each
-// swapping the off-diagonal s x s blocks between lanes k and k ^ s.
-__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t masks[5] = { 0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u };
-#pragma unroll
-    for (int i = 0; i < 5; i++) {
-        const uint32_t s = 16u >> i, m = masks[i];
-        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, (int)s);
-        x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
-    }
-    return x;
 }
 
 // GEN: a target is not RGBA / unsigned byte.  PHONG: a draw state lights per
