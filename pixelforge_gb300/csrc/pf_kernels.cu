@@ -146,13 +146,18 @@ __device__ __forceinline__ uint32_t pack4(const int32_t *v)
 // blend.h:140-277 (SUB adds; channels are ORed without masks when packed)
 __device__ uint32_t blend_simd(int mode, uint32_t src, uint32_t dst)
 {
+    if (mode == 1) {
+        // alpha: (s a + d (256 - a)) >> 8 a channel, the source's alpha taken
+        // as 255, two channels a multiply (a sum stays below 2^16)
+        const uint32_t a = (src >> 24) + 1u, ia = 256u - a;
+        const uint32_t rb = (src & 0x00ff00ffu) * a + (dst & 0x00ff00ffu) * ia;
+        const uint32_t ga = (((src >> 8) & 0x000000ffu) | 0x00ff0000u) * a + ((dst >> 8) & 0x00ff00ffu) * ia;
+        return ((rb >> 8) & 0x00ff00ffu) | (ga & 0xff00ff00u);
+    }
     int32_t s[4], d[4], o[4];
     for (int i = 0; i < 4; i++) { s[i] = (int32_t)chn(src, i); d[i] = (int32_t)chn(dst, i); }
     switch (mode) {
     case 0: for (int i = 0; i < 4; i++) o[i] = (s[i] + d[i]) >> 1; break;
-    case 1: { int32_t a = s[3] + 1, ia = 256 - a;
-              for (int i = 0; i < 3; i++) o[i] = (s[i]*a + d[i]*ia) >> 8;
-              o[3] = (255*a + d[3]*ia) >> 8; } break;
     case 2: for (int i = 0; i < 4; i++) { int32_t t = s[i] + d[i]; o[i] = t < 255 ? t : 255; } break;
     case 3: for (int i = 0; i < 4; i++) { int32_t t = s[i] + d[i]; o[i] = t > 0 ? t : 0; } break;
     case 4: for (int i = 0; i < 4; i++) o[i] = (s[i]*d[i]) >> 8; break;
@@ -2032,8 +2037,8 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// k_rows: targets of BGRA / unsigned-byte format, band by band in
-// submission order.
+// k_rows: targets of BGRA / unsigned-byte format, row by row in submission
+// order.
 //
 // The reference writes such a framebuffer through a SIMD getter and setter
 // that shuffle each 4-pixel half of the 8-pixel vector with the bytes of
@@ -2045,32 +2050,73 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
 // the triangle's box (x steps by 8 from xMin, triangles.c:409), so a half's
 // first pixel may lie in the tile to the left, whose colour when the
 // triangle is drawn depends on everything drawn there before it: the tiles
-// of a row are not independent.  Rows are.  A warp owns one row of such a
-// target for the whole launch and walks the launch's items in submission
-// order -- four 8-byte summaries a lane at a time (row_info: the records an
-// item has and the rows they span), so that items off the row cost a
-// coalesced load -- drawing each record whose box meets the row: its
-// 4-pixel halves are spread over the lanes, each lane drawing its half
-// alone, and the warp moves to the next record when all are done.  Points,
-// lines and rectangles use the scalar getter and setter (a plain R / B
-// swap, pixel.h:356-363, 703-707), pixel by pixel.
+// of a row are not independent.  Rows are.  Points, lines and rectangles use
+// the scalar getter and setter (a plain R / B swap, pixel.h:356-363,
+// 703-707), pixel by pixel.
+//
+// A CTA owns one row of such a target for the whole launch and keeps its
+// colour and depth in shared memory.  Only the depth test and the blend need
+// the row as it is when a record is drawn; a half's coverage, its pixels'
+// depths and both colours its first pixel can give (inside the mask or
+// outside) do not.  So the row's records pass through a pipeline, a batch of
+// up to 32 records a step, one block barrier between steps: one warp looks
+// for records that reach the row (8-byte summaries -- row_info: the records
+// an item has and the rows they span -- so that items off the row cost a
+// coalesced load), one makes the next batch and loads its records, two work
+// out the halves of the batch before, and one draws the batch before that,
+// record by record, a lane a pixel.  Bound by that last chain: a record's
+// step reads its pixels, compares, blends and writes.  With one warp doing
+// all of it a record at a time (its load and its texels waited for in every
+// step) the sphere frame's launch at 1080p took 800 us; with a lane a half
+// in the drawing warp and one finding warp 240; this takes 177 us.
 // ---------------------------------------------------------------------------
-#define ROW_WARPS 4
+#define ROW_THREADS 160
+#define ROW_BATCH 32                // records of a batch
+#define ROW_HALVES 96               // halves of a batch (a wider record is drawn in parts)
+#define ROW_AHEAD 128               // records the looking warp keeps in the queue
+#define ROW_QUEUE 2048              // its room: those and what four groups of 32 items may add
 
-// One record over row y of a BGRA / unsigned-byte target of width W whose
-// colour and depth the row pointers crow / drow hold (in global or shared
-// memory), the part of lane `lane`; returns the covered pixels it counted.
-__device__ __noinline__ uint32_t row_record(const PFPrim &P, const PFPrimPhong *ph, const PFDrawState *states,
-                                            uint32_t *crow, float *drow, uint32_t W, uint32_t y, uint32_t lane)
+struct __align__(16) RowHalf {
+    float z[4];                     // its pixels' depths
+    uint32_t cov;                   // bit j: pixel j is covered
+    uint32_t in, out;               // its colour when its first pixel passes, and when it does not
+    uint32_t pad;                   // (R and B swapped as they are stored, but for modes that blend in RGBA order)
+};
+struct __align__(16) RowEntry {
+    uint32_t x;                     // first pixel of its first half in the batch
+    uint32_t n;                     // halves | place of the first in the batch << 8 | kind << 16
+    uint32_t rstate;
+    uint32_t ref;                   // item, or pool index with the top bit
+};
+struct RowShared {
+    SPrim rec[2][ROW_BATCH];
+    RowHalf half[2][ROW_HALVES];
+    RowEntry entry[3][ROW_BATCH];
+    uint32_t queue[ROW_QUEUE];
+    uint32_t nEntries[3], nHalves[3];
+    uint32_t tail[2], head[2];      // of the queue, as of the last steps
+    uint32_t found[2];              // whether nothing more comes
+    uint32_t last;                  // the step that made the last batch
+};
+static_assert(ROW_AHEAD + 4 * 32 * PF_MAX_SUBTRIS <= ROW_QUEUE && (ROW_QUEUE & (ROW_QUEUE - 1)) == 0, "room for four groups' records");
+static_assert(ROW_HALVES < 256 && PFP_KIND < 256, "fields of RowEntry.n");
+
+// Blending in the stored order is the same for the modes that treat R and B
+// alike: none, and alpha.  (SUB's channels are ORed without masks.)
+__device__ __forceinline__ bool row_swapped(uint32_t rs) { return !(rs & PFS_BLEND) || (rs >> 24) == 1u; }
+
+__device__ __forceinline__ const PFPrim *row_prim(const RasterArgs &a, uint32_t ref)
 {
-    // the row and columns as tile_edge clips a box: y in [yMin, yMax], x in
-    // [xMin, xMax), inside the framebuffer (unsigned)
-    const uint32_t xMin = (uint32_t)P.xMin, xMax = (uint32_t)P.xMax, yMin = (uint32_t)P.yMin, yMax = (uint32_t)P.yMax;
-    const uint32_t xEnd = min(xMax, W);
-    if (xMin >= xEnd || y < yMin || y > yMax) return 0;
-    const uint32_t nH = (xEnd - xMin + 3u) / 4u;
-    const uint32_t kind = P.flags & PFP_KIND, rs = P.rstate;
-    const int func = (int)((rs >> 16) & 255u), mode = (int)(rs >> 24);
+    return (ref & 0x80000000u) ? a.pool + (ref & 0x7fffffffu) : a.prims + ref;
+}
+
+// Half (xf, y) of a set-up triangle: everything that does not depend on the
+// row's contents.  Returns the covered pixels.
+template <bool PHONG>
+__device__ __forceinline__ uint32_t row_half(const SPrim &R, const PFDrawState *states, uint32_t xf, uint32_t y, uint32_t W, RowHalf &H)
+{
+    const PFPrim &P = R.p;
+    const uint32_t xEnd = min((uint32_t)P.xMax, W), rs = P.rstate;
     // edge functions at pixel (x, y): (x - rx) sx + (y - ry) sy, 32-bit
     // wrapping (triangles.c:336-349, 398-420)
     int32_t sx[3] = { P.y3 - P.y2, P.y1 - P.y3, P.y2 - P.y1 };
@@ -2078,71 +2124,206 @@ __device__ __noinline__ uint32_t row_record(const PFPrim &P, const PFPrimPhong *
     const int32_t rx[3] = { P.x2, P.x3, P.x1 }, ry[3] = { P.y2, P.y3, P.y1 };
     if (P.flags & 1u)
         for (int e = 0; e < 3; e++) { sx[e] = -sx[e]; sy[e] = -sy[e]; }
+    uint32_t w[3];
+    for (int e = 0; e < 3; e++)
+        w[e] = (xf - (uint32_t)rx[e]) * (uint32_t)sx[e] + (y - (uint32_t)ry[e]) * (uint32_t)sy[e];
+    float wf[3] = { 0.0f, 0.0f, 0.0f }, zl[4];
     uint32_t cov = 0;
-    for (uint32_t t = lane; t < nH; t += 32) {
-        const uint32_t xf = xMin + 4u * t;
-        if (kind == 0) {
-            bool m[4] = { false, false, false, false }, any = false;
-            float zl[4] = { 0.0f, 0.0f, 0.0f, 0.0f }, wf[3] = { 0.0f, 0.0f, 0.0f }, zf = 0.0f;
-            for (uint32_t j = 0; j < 4; j++) {
-                const uint32_t x = xf + j;
-                uint32_t w[3];
-                for (int e = 0; e < 3; e++)
-                    w[e] = (x - (uint32_t)rx[e]) * (uint32_t)sx[e] + (y - (uint32_t)ry[e]) * (uint32_t)sy[e];
-                const float wn1 = (float)(int32_t)w[0] * P.wInvSum, wn2 = (float)(int32_t)w[1] * P.wInvSum;
-                const float wn3 = (float)(int32_t)w[2] * P.wInvSum;
-                float zs = P.z1 * wn1 + P.z2 * wn2;
-                zs = zs + P.z3 * wn3;
-                const float z = __frcp_rn(zs);
-                if (j == 0) { wf[0] = wn1; wf[1] = wn2; wf[2] = wn3; zf = z; }
-                if (x >= xEnd || (int32_t)(w[0] | w[1] | w[2]) <= 0) continue;
-                cov++;
-                if ((rs & PFS_DEPTH_TEST) && !depth_simd(func, z, drow[x])) continue;
-                m[j] = true; zl[j] = z; any = true;
-            }
-            if (!any) continue;
-            // the half's value: its first pixel's colour and destination
-            uint32_t frag = shade_fragment<true>(P, ph, states, wf[0], wf[1], wf[2], zf, m[0], true);
-            if (rs & PFS_BLEND) frag = blend_simd(mode, frag, pff_swap_rb(crow[xf]));
-            const uint32_t out = pff_swap_rb(frag);
-            for (uint32_t j = 0; j < 4; j++) {
-                if (!m[j]) continue;
-                crow[xf + j] = out;
-                if (rs & PFS_DEPTH_MASK) drow[xf + j] = zl[j];
-            }
-        } else {
-            for (uint32_t j = 0; j < 4; j++) {
-                const uint32_t x = xf + j;
-                if (x >= xEnd || !lp_covers(P, (int32_t)x, (int32_t)y)) continue;
-                if (kind != PFP_BLIT) cov++;
-                const float z = lp_depth(P, (int32_t)x, (int32_t)y);
-                if ((rs & PFS_DEPTH_TEST) && !depth_sisd(func, z, drow[x])) continue;
-                uint32_t c = lp_color(P, (int32_t)x, (int32_t)y);
-                if (rs & PFS_BLEND) c = blend_sisd(mode, c, pff_swap_rb(crow[x]));
-                crow[x] = pff_swap_rb(c);
-                if (rs & PFS_DEPTH_MASK) drow[x] = z;
-            }
-        }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        const float wn1 = (float)(int32_t)w[0] * P.wInvSum, wn2 = (float)(int32_t)w[1] * P.wInvSum;
+        const float wn3 = (float)(int32_t)w[2] * P.wInvSum;
+        float zs = P.z1 * wn1 + P.z2 * wn2;
+        zs = zs + P.z3 * wn3;
+        zl[j] = __frcp_rn(zs);
+        if (j == 0) { wf[0] = wn1; wf[1] = wn2; wf[2] = wn3; }
+        if (xf + j < xEnd && (int32_t)(w[0] | w[1] | w[2]) > 0) cov |= 1u << j;
+        for (int e = 0; e < 3; e++) w[e] += (uint32_t)sx[e];
+    }
+    H.z[0] = zl[0]; H.z[1] = zl[1]; H.z[2] = zl[2]; H.z[3] = zl[3];
+    H.cov = cov;
+    if (cov) {
+        // the colours of the outcomes there can be: the first pixel outside
+        // the mask unless it is covered and no depth test can take it out
+        const bool in = (cov & 1u) != 0, out = !in || (rs & PFS_DEPTH_TEST);
+        uint32_t c = 0;
+        if (in) c = shade_fragment<PHONG>(P, R.ph, states, wf[0], wf[1], wf[2], zl[0], true, true);
+        H.in = row_swapped(rs) ? pff_swap_rb(c) : c;
+        if (out && (!in || (rs & PFS_TEXTURE))) c = shade_fragment<PHONG>(P, R.ph, states, wf[0], wf[1], wf[2], zl[0], false, true);
+        H.out = row_swapped(rs) ? pff_swap_rb(c) : c;
+    }
+    return (uint32_t)__popc(cov);
+}
+
+// The pixels of a row, colour and depth bits: in shared memory, or in place.
+template <bool SMEM> struct RowPixels;
+template <> struct RowPixels<true> {
+    uint2 *p;
+    __device__ __forceinline__ uint2 get(uint32_t x) const { return p[x]; }
+    __device__ __forceinline__ void set(uint32_t x, uint32_t c, uint32_t d) const { p[x] = make_uint2(c, d); }
+};
+template <> struct RowPixels<false> {
+    uint32_t *c;
+    float *d;
+    __device__ __forceinline__ uint2 get(uint32_t x) const { return make_uint2(c[x], __float_as_uint(d[x])); }
+    __device__ __forceinline__ void set(uint32_t x, uint32_t cv, uint32_t dv) const { c[x] = cv; d[x] = __uint_as_float(dv); }
+};
+
+// A point, line or rectangle over n halves of row y from pixel x on; returns
+// the fragments it counted.
+template <bool SMEM>
+__device__ __noinline__ uint32_t row_scalar(const PFPrim &P, uint32_t rs, uint32_t x0, uint32_t n, RowPixels<SMEM> row,
+                                            uint32_t W, uint32_t y, uint32_t lane)
+{
+    const uint32_t xEnd = min(min((uint32_t)P.xMax, W), x0 + 4u * n);
+    uint32_t cov = 0;
+    for (uint32_t x = x0 + lane; x < xEnd; x += 32) {
+        if (!lp_covers(P, (int32_t)x, (int32_t)y)) continue;
+        if ((P.flags & PFP_KIND) != PFP_BLIT) cov++;
+        const float z = lp_depth(P, (int32_t)x, (int32_t)y);
+        const uint2 p = row.get(x);
+        if ((rs & PFS_DEPTH_TEST) && !depth_sisd((int)((rs >> 16) & 255u), z, __uint_as_float(p.y))) continue;
+        uint32_t c = lp_color(P, (int32_t)x, (int32_t)y);
+        if (rs & PFS_BLEND) c = blend_sisd((int)(rs >> 24), c, pff_swap_rb(p.x));
+        row.set(x, pff_swap_rb(c), (rs & PFS_DEPTH_MASK) ? __float_as_uint(z) : p.y);
     }
     return cov;
 }
 
-// SMEM: the warp keeps its row's colour and depth in shared memory while it
-// draws (rows up to ROW_SMEM_MAX_W pixels), else it draws in place.
+// The warp that looks for the row's records, in order.
+struct RowFinder {
+    int si;                         // segment
+    uint32_t gBegin, gEnd;          // its items
+    uint32_t cb, cEnd;              // next group of 32 items to look at
+    uint32_t base, m[4];            // groups that reach the row, of the 128 from base on
+    uint32_t tail;                  // of the queue
+    bool done;                      // no group left
+};
+
+__device__ __forceinline__ bool on_row(uint64_t w, uint64_t some, uint32_t y)
+{
+    return (w & some) && ((w >> 16) & 0xffffffu) <= y && (w >> 40) >= y;
+}
+
+// Puts records that may reach row y of target t on the queue until it holds
+// ROW_AHEAD.  The whole warp calls it.
+__device__ __forceinline__ void row_find(const RasterArgs &a, RowFinder &F, RowShared &S, const PFSegment *__restrict__ segs, int nSegs,
+                                         const uint64_t *__restrict__ rowInfo, const uint64_t *__restrict__ rowGroup,
+                                         int t, uint32_t y, uint32_t head)
+{
+    const uint32_t lane = threadIdx.x & 31u, all = 0xffffffffu;
+    while (F.tail - head < (uint32_t)ROW_AHEAD && !F.done) {
+        if (!(F.m[0] | F.m[1] | F.m[2] | F.m[3])) {
+            // the next 128 groups
+            while (F.cb >= F.cEnd && !F.done) {
+                do F.si++; while (F.si < nSegs && (segs[F.si].target != t || segs[F.si].nItems == 0));
+                if (F.si >= nSegs) { F.done = true; break; }
+                F.gBegin = segs[F.si].itemBase; F.gEnd = F.gBegin + segs[F.si].nItems;
+                F.cb = F.gBegin >> 5; F.cEnd = ((F.gEnd - 1u) >> 5) + 1u;
+            }
+            if (F.done) break;
+            uint64_t w[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) { const uint32_t c = F.cb + 32u * i + lane; w[i] = c < F.cEnd ? __ldg(rowGroup + c) : 0ull; }
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) F.m[i] = __ballot_sync(all, on_row(w[i], 1ull, y));
+            F.base = F.cb;
+            F.cb += 128u;
+            continue;
+        }
+        // the items' records of the next four groups that may reach the row
+        // (four loads under way instead of one)
+        uint32_t g[4];
+        uint64_t w[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) {
+            uint32_t at = 0xffffffffu;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++)
+                if (at == 0xffffffffu && F.m[i]) {
+                    at = F.base + 32u * i + (uint32_t)(__ffs(F.m[i]) - 1);
+                    F.m[i] &= F.m[i] - 1u;
+                }
+            g[q] = at == 0xffffffffu ? 0xffffffffu : (at << 5) + lane;
+            w[q] = (g[q] >= F.gBegin && g[q] < F.gEnd) ? __ldg(rowInfo + g[q]) : 0ull;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) {
+            const uint32_t subs = on_row(w[q], 0xffffull, y) ? (uint32_t)w[q] & 0xffffu : 0u;
+            uint32_t total;
+            uint32_t at = F.tail + warp_offsets((uint32_t)__popc(subs), total);
+            const uint32_t pb = (subs & ~1u) ? (uint32_t)__ldg(&a.prims[g[q]].poolBase) : 0u;
+            for (uint32_t mm = subs; mm; mm &= mm - 1u, at++) {
+                const uint32_t sub = (uint32_t)(__ffs(mm) - 1);
+                S.queue[at & (ROW_QUEUE - 1)] = sub ? 0x80000000u | (pb + sub - 1u) : g[q];
+            }
+            F.tail += total;
+        }
+    }
+}
+
+// Makes the next batch of row y from the queue's records [head, tail) and
+// loads its records into slot `step` of the buffers; part: halves of the
+// first one that are in an earlier batch.  The whole warp calls it.
+template <bool PHONG>
+__device__ __forceinline__ void row_batch(const RasterArgs &a, RowShared &S, uint32_t &head, uint32_t tail, uint32_t &part, bool found,
+                                          uint32_t W, uint32_t y, uint32_t step)
+{
+    const uint32_t lane = threadIdx.x & 31u, all = 0xffffffffu;
+    // whole records while their halves fit, and part of the next
+    const uint32_t n = min((uint32_t)ROW_BATCH, tail - head);
+    uint32_t ref = 0, x = 0, len = 0, rs = 0, kind = 0;
+    const uint32_t t0 = lane == 0 ? part : 0u;
+    if (lane < n) {
+        ref = S.queue[(head + lane) & (ROW_QUEUE - 1)];
+        SPrim &R = S.rec[step & 1u][lane];
+        const int4 *src = reinterpret_cast<const int4 *>(row_prim(a, ref));
+        int4 r[8];
+        for (int i = 0; i < 8; i++) r[i] = __ldg(src + i);
+        for (int i = 0; i < 8; i++) reinterpret_cast<int4 *>(&R.p)[i] = r[i];
+        if (PHONG) R.ph = (ref & 0x80000000u) ? a.poolPh + (ref & 0x7fffffffu) : a.primsPh + ref;
+        rs = (uint32_t)r[4].w; kind = (uint32_t)r[2].z & PFP_KIND;
+        // the row and columns as tile_edge clips a box: y in [yMin, yMax], x
+        // in [xMin, xMax), inside the framebuffer (unsigned)
+        const uint32_t xMin = (uint32_t)r[1].z, xEnd = min((uint32_t)r[2].x, W);
+        if (xMin < xEnd && y >= (uint32_t)r[1].w && y <= (uint32_t)r[2].y) {
+            len = (xEnd - xMin + 3u) / 4u - t0;
+            x = xMin + 4u * t0;
+        }
+    }
+    uint32_t total;
+    const uint32_t h0 = warp_offsets(min(len, (uint32_t)ROW_HALVES + 1u), total);
+    const uint32_t fit = h0 >= (uint32_t)ROW_HALVES ? 0u : min(len, (uint32_t)ROW_HALVES - h0);
+    const uint32_t over = __ballot_sync(all, lane < n && fit < len);
+    const uint32_t whole = over ? (uint32_t)(__ffs(over) - 1) : n;             // records finished by this batch
+    uint32_t cut = __shfl_sync(all, fit, (int)(whole & 31u));
+    if (!over) cut = 0u;                                                        // halves taken of the next
+    const uint32_t entries = whole + (cut ? 1u : 0u), s3 = step % 3u;
+    if (lane < entries) S.entry[s3][lane] = RowEntry{ x, fit | h0 << 8 | kind << 16, rs, ref };
+    const uint32_t end = __shfl_sync(all, h0 + fit, (int)((entries - 1u) & 31u));
+    part = over ? (whole == 0 ? part : 0u) + cut : 0u;
+    head += whole;
+    if (lane == 0) {
+        S.nEntries[s3] = entries; S.nHalves[s3] = entries ? end : 0u;
+        if (found && head == tail) S.last = step;
+    }
+}
+
+// SMEM: the row's colour and depth are kept in shared memory (rows up to
+// ROW_SMEM_MAX_W pixels), else they are drawn in place.
 #define ROW_SMEM_MAX_W 2048
-template <bool SMEM>
-__global__ void __launch_bounds__(ROW_WARPS * 32) k_rows(RasterArgs a, const PFSegment *__restrict__ segs, int nSegs,
+template <bool SMEM, bool PHONG>
+__global__ void __launch_bounds__(ROW_THREADS, 5) k_rows(RasterArgs a, const PFSegment *__restrict__ segs, int nSegs,
                                                          const uint64_t *__restrict__ rowInfo,
-                                                         const uint64_t *__restrict__ rowGroup, uint32_t nRows)
+                                                         const uint64_t *__restrict__ rowGroup, uint32_t rowW)
 {
     extern __shared__ __align__(16) unsigned char rowSmem[];
-    __shared__ __align__(16) PFPrim sRec[ROW_WARPS];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    RowShared &S = *reinterpret_cast<RowShared *>(rowSmem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // k_raster is done
     if (a.cnt->abortCommand <= a.command) return;
     // my row: row y of the BGRA / unsigned-byte targets, in target order
-    uint32_t y = blockIdx.x * ROW_WARPS + warp;
-    if (y >= nRows) return;
+    uint32_t y = blockIdx.x;
     int t = 0;
     for (; t < a.nTargets; t++) {
         if (a.targets[t].fmt != PFF_BGRA8) continue;
@@ -2154,59 +2335,123 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) k_rows(RasterArgs a, const PFS
     const uint32_t W = T.W;
     uint32_t *gcol = static_cast<uint32_t *>(T.color) + (size_t)y * W;
     float *gdep = T.depth + (size_t)y * W;
-    uint32_t *crow = gcol;
-    float *drow = gdep;
-    if (SMEM) {
-        crow = reinterpret_cast<uint32_t *>(rowSmem) + (size_t)warp * 2 * ROW_SMEM_MAX_W;
-        drow = reinterpret_cast<float *>(crow + ROW_SMEM_MAX_W);
-    }
+    RowPixels<SMEM> row;
+    if constexpr (SMEM) row.p = reinterpret_cast<uint2 *>(rowSmem + sizeof(RowShared));
+    else { row.c = gcol; row.d = gdep; }
     // the row as the draws find it: the fused clear (pfClear keeps pixels
     // 0..7), or the framebuffer's contents
-    for (uint32_t x = lane; x < W; x += 32) {
+    for (uint32_t x = tid; x < W; x += ROW_THREADS) {
         const bool clr = T.clearMode == 2 || (T.clearMode == 1 && (size_t)y * W + x >= 8);
-        if (clr) { crow[x] = T.clearRaw[0]; drow[x] = T.clearDepth; }
-        else if (SMEM) { crow[x] = gcol[x]; drow[x] = gdep[x]; }
+        if (clr) row.set(x, T.clearRaw[0], __float_as_uint(T.clearDepth));
+        else if (SMEM) row.set(x, gcol[x], __float_as_uint(gdep[x]));
     }
-    __syncwarp();
-    PFPrim &R = sRec[warp];
+    if (tid == 0) {
+        S.last = 0xffffffffu;
+        for (int i = 0; i < 2; i++) S.head[i] = S.tail[i] = S.found[i] = 0u;
+    }
+    __syncthreads();
+    RowFinder F{ -1, 0, 0, 0, 0, 0, { 0, 0, 0, 0 }, 0, false };
+    uint32_t head = 0, part = 0;
     unsigned long long frags = 0;
-    for (int si = 0; si < nSegs; si++) {
-        if (segs[si].target != t) continue;
-        const uint32_t gBegin = segs[si].itemBase, gEnd = gBegin + segs[si].nItems;
-        if (gBegin >= gEnd) continue;
-        // groups of 32 items (one summary word each, 32 groups a step), then
-        // the items of the groups that reach the row, in order
-        const uint32_t cEnd = ((gEnd - 1) >> 5) + 1;
-        for (uint32_t cb = gBegin >> 5; cb < cEnd; cb += 32) {
-            const uint32_t c = cb + lane;
-            const uint64_t sg = c < cEnd ? __ldg(rowGroup + c) : 0ull;
-            const bool ghit = (sg & 1u) && ((sg >> 16) & 0xffffffu) <= y && (sg >> 40) >= y;
-            for (uint32_t gneed = __ballot_sync(0xffffffffu, ghit); gneed; gneed &= gneed - 1) {
-                const uint32_t gb = (cb + (uint32_t)(__ffs(gneed) - 1)) << 5;
-                const uint32_t g = gb + lane;
-                const uint64_t w = (g >= gBegin && g < gEnd) ? __ldg(rowInfo + g) : 0ull;
-                const bool hit = (w & 0xffffu) && ((w >> 16) & 0xffffffu) <= y && (w >> 40) >= y;
-                for (uint32_t need = __ballot_sync(0xffffffffu, hit); need; need &= need - 1) {
-                    const int src = __ffs(need) - 1;
-                    const uint32_t gi = gb + (uint32_t)src;
-                    const uint32_t subs = (uint32_t)__shfl_sync(0xffffffffu, (uint32_t)w, src) & 0xffffu;
-                    const int32_t pb = (subs & ~1u) ? __ldg(&a.prims[gi].poolBase) : 0;
-                    for (uint32_t mm = subs; mm; mm &= mm - 1) {
-                        const uint32_t sub = (uint32_t)(__ffs(mm) - 1);
-                        const uint32_t pi = sub ? (uint32_t)pb + sub - 1 : gi;
-                        const PFPrim *rec = sub ? &a.pool[pi] : &a.prims[gi];
-                        if (lane < 8) reinterpret_cast<int4 *>(&R)[lane] = __ldg(reinterpret_cast<const int4 *>(rec) + lane);
-                        __syncwarp();
-                        const PFPrimPhong *ph = a.anyPhong ? (sub ? &a.poolPh[pi] : &a.primsPh[gi]) : nullptr;
-                        frags += row_record(R, ph, a.states, crow, drow, W, y, lane);
-                        __syncwarp();              // the record's pixels are written; R is free
-                    }
+    // step s looks ahead, makes batch s of the records found before it, works
+    // out the halves of batch s - 1 and draws batch s - 2
+    for (uint32_t step = 0;; step++) {
+        const uint32_t last = S.last;                      // (this step may write it: nothing differs before two steps on)
+        if (last != 0xffffffffu && step > last + 2u) break;
+        if (warp == 4) {
+            if (!S.found[(step + 1u) & 1u]) row_find(a, F, S, segs, nSegs, rowInfo, rowGroup, t, y, S.head[(step + 1u) & 1u]);
+            __syncwarp();
+            if (lane == 0) { S.tail[step & 1u] = F.tail; S.found[step & 1u] = F.done; }
+        } else if (warp == 1) {
+            if (last == 0xffffffffu)
+                row_batch<PHONG>(a, S, head, S.tail[(step + 1u) & 1u], part, S.found[(step + 1u) & 1u] != 0, W, y, step);
+            if (lane == 0) S.head[step & 1u] = head;
+        } else if (warp >= 2) {
+            if (step >= 1 && step - 1u <= last) {
+                const uint32_t b = step - 1u, nE = S.nEntries[b % 3u], nH = S.nHalves[b % 3u];
+                const RowEntry *E = S.entry[b % 3u];
+                for (uint32_t h = tid - 64u; h < nH; h += 64u) {
+                    // its entry: the last one that starts at or before it
+                    uint32_t lo = 0, hi = nE - 1u;
+                    while (lo < hi) { const uint32_t mid = (lo + hi + 1u) >> 1; if (((E[mid].n >> 8) & 255u) <= h) lo = mid; else hi = mid - 1u; }
+                    const RowEntry e = E[lo];
+                    if (!(e.n >> 16))
+                        frags += row_half<PHONG>(S.rec[b & 1u][lo], a.states, e.x + 4u * (h - ((e.n >> 8) & 255u)), y, W, S.half[b & 1u][h]);
                 }
             }
+        } else if (step >= 2 && step - 2u <= last) {
+            const uint32_t b = step - 2u, nE = S.nEntries[b % 3u];
+            const RowEntry *E = S.entry[b % 3u];
+            const RowHalf *H = S.half[b & 1u];
+            // a lane a pixel, eight halves at a time; the next record's entry
+            // and halves are read while one is drawn.  A lane reads and
+            // writes its own pixel only: the first pixel's colour and its
+            // outcome come from its lane.
+            const uint32_t j = lane & 3u, k0 = lane >> 2, quad = lane & 28u;
+            RowEntry e{};
+            float z = 0.0f;
+            uint4 c = make_uint4(0, 0, 0, 0);                  // cov, in, out
+            auto fetch = [&](uint32_t i, RowEntry &en, float &zn, uint4 &cn) {
+                en.n = 0;
+                cn.x = 0;
+                if (i < nE) {
+                    en = E[i];
+                    if (k0 < (en.n & 255u) && !(en.n >> 16)) {
+                        const RowHalf &h = H[((en.n >> 8) & 255u) + k0];
+                        zn = h.z[j];
+                        cn = *reinterpret_cast<const uint4 *>(&h.cov);
+                    }
+                }
+            };
+            fetch(0, e, z, c);
+            for (uint32_t i = 0; i < nE; i++) {
+                RowEntry en;
+                float zn = 0.0f;
+                uint4 cn;
+                fetch(i + 1u, en, zn, cn);
+                const uint32_t rs = e.rstate, n = e.n & 255u;
+                if (e.n >> 16) {
+                    frags += row_scalar<SMEM>(*row_prim(a, e.ref), rs, e.x, n, row, W, y, lane);
+                } else {
+                    for (uint32_t h = 0;;) {
+                        const uint32_t x = e.x + 4u * (h + k0) + j;
+                        uint2 p = make_uint2(0, 0);
+                        if (c.x && x < W) p = row.get(x);
+                        bool pass = (c.x >> j) & 1u;
+                        if (rs & PFS_DEPTH_TEST) {
+                            const uint32_t func = (rs >> 16) & 255u;
+                            const float d = __uint_as_float(p.y);
+                            pass = pass && (func == 2u ? z < d : depth_simd((int)func, z, d));
+                        }
+                        const uint32_t m = __ballot_sync(0xffffffffu, pass) >> quad;
+                        // the half's value: its first pixel's colour and destination
+                        uint32_t frag = (m & 1u) ? c.y : c.z;
+                        if (rs & PFS_BLEND) {
+                            const uint32_t dst = __shfl_sync(0xffffffffu, p.x, (int)quad);
+                            const uint32_t mode = rs >> 24;
+                            frag = mode == 1u ? blend_simd(1, frag, dst) : pff_swap_rb(blend_simd((int)mode, frag, pff_swap_rb(dst)));
+                        }
+                        if (pass) row.set(x, frag, (rs & PFS_DEPTH_MASK) ? __float_as_uint(z) : p.y);
+                        h += 8u;
+                        if (h >= n) break;
+                        c.x = 0;                               // (more than eight halves)
+                        if (h + k0 < n) {
+                            const RowHalf &q = H[((e.n >> 8) & 255u) + h + k0];
+                            z = q.z[j];
+                            c = *reinterpret_cast<const uint4 *>(&q.cov);
+                        }
+                    }
+                }
+                __syncwarp();                                  // the record's pixels are written
+                e = en;
+                z = zn;
+                c = cn;
+            }
         }
+        __syncthreads();
     }
     if (SMEM)
-        for (uint32_t x = lane; x < W; x += 32) { gcol[x] = crow[x]; gdep[x] = drow[x]; }
+        for (uint32_t x = tid; x < W; x += ROW_THREADS) { const uint2 p = row.get(x); gcol[x] = p.x; gdep[x] = __uint_as_float(p.y); }
     for (int o = 16; o > 0; o >>= 1) frags += __shfl_down_sync(0xffffffffu, frags, o);
     if (lane == 0 && frags) atomicAdd(&a.cnt->fragments, frags);
 }
@@ -2460,16 +2705,15 @@ cudaError_t pfd_launch_raster(const PFBatchLaunch &L, cudaStream_t st)
     if (e != cudaSuccess) return e;
     e = launch_serialized(kernel, grid, (unsigned)(warps * 32), smem, st, raster_args(L));
     if (e != cudaSuccess || L.rowCount == 0 || !L.rowInfo || !L.rowGroup) return e;
-    const unsigned rowGrid = (L.rowCount + ROW_WARPS - 1) / ROW_WARPS;
-    if (L.rowMaxW <= ROW_SMEM_MAX_W) {
-        const size_t rsm = (size_t)ROW_WARPS * 2 * ROW_SMEM_MAX_W * 4;          // colour and depth rows
-        e = cudaFuncSetAttribute(k_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
-        if (e != cudaSuccess) return e;
-        return launch_serialized(k_rows<true>, rowGrid, ROW_WARPS * 32, rsm, st, raster_args(L), L.segs, L.nSegs,
-                                 (const uint64_t *)L.rowInfo, (const uint64_t *)L.rowGroup, L.rowCount);
-    }
-    return launch_serialized(k_rows<false>, rowGrid, ROW_WARPS * 32, 0, st, raster_args(L), L.segs, L.nSegs,
-                             (const uint64_t *)L.rowInfo, (const uint64_t *)L.rowGroup, L.rowCount);
+    const bool inSmem = L.rowMaxW <= ROW_SMEM_MAX_W;
+    const uint32_t rowW = (L.rowMaxW + 3u) & ~3u;
+    const size_t rsm = sizeof(RowShared) + (inSmem ? (size_t)rowW * 8 : 0);            // colour and depth of the row
+    auto rows = inSmem ? (L.anyPhong ? k_rows<true, true> : k_rows<true, false>)
+                       : (L.anyPhong ? k_rows<false, true> : k_rows<false, false>);
+    e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
+    if (e != cudaSuccess) return e;
+    return launch_serialized(rows, L.rowCount, ROW_THREADS, rsm, st, raster_args(L), L.segs, L.nSegs,
+                             (const uint64_t *)L.rowInfo, (const uint64_t *)L.rowGroup, rowW);
 }
 
 cudaError_t pfd_launch_clear(void *color, uint32_t fmt, float *depth, size_t n, const uint32_t cc[4], float cd, bool all,
