@@ -1626,7 +1626,10 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
     // is then two work items, its top and bottom halves, each a warp with
     // one pixel a lane, which take about half as long.  Where heavy tiles
     // are many the launch is bound by the total work, which halves would
-    // only add to (each half walks the whole bin).
+    // only add to (each half walks the whole bin).  A launch of at most half
+    // as many tiles as warps has idle warps for every level (the 64 tiles of
+    // a 64x64 context 57 -> 31 us, the 1,024 of soup256 56 -> 50; taking
+    // halves of all levels up to half the warps instead, phong1080 335 -> 357).
     // (in shared memory, like the fragment count: read by lane 0 between
     // tiles only, they would cost the tile's loops registers)
     __shared__ uint32_t sLevelEnd[PF_HEAVY_LEVELS + 1];    // queue index past level l's entries, heaviest first
@@ -1636,7 +1639,7 @@ __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
         uint32_t nQueue = 0, split = 0;
         for (int l = PF_HEAVY_LEVELS; l >= 1; l--) {
             const uint32_t c = min(a.cnt->heavyCount[l - 1], a.totalTiles);
-            const bool sp = 4u * c <= gridDim.x * (uint32_t)WARPS;
+            const bool sp = 4u * c <= gridDim.x * (uint32_t)WARPS || 2u * a.totalTiles <= gridDim.x * (uint32_t)WARPS;
             split |= sp ? 1u << l : 0u;
             nQueue += sp ? 2u * c : c;
             sLevelEnd[l] = nQueue;
@@ -2716,7 +2719,7 @@ cudaError_t pfd_launch_raster(const PFBatchLaunch &L, cudaStream_t st)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     uint32_t grid = 0;
     if (e == cudaSuccess) e = persistent_grid((const void *)kernel, warps * 32, smem, L.rasterCtasPerSM,
-                                              (L.totalTiles + (uint32_t)warps - 1) / (uint32_t)warps, grid);
+                                              (2u * L.totalTiles + (uint32_t)warps - 1) / (uint32_t)warps, grid);  // half tiles
     if (e != cudaSuccess) return e;
     e = launch_serialized(kernel, grid, (unsigned)(warps * 32), smem, st, raster_args(L));
     if (e != cudaSuccess || L.rowCount == 0 || !L.rowInfo || !L.rowGroup) return e;
