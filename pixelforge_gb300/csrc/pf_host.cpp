@@ -295,7 +295,8 @@ struct Renderer {
     // device
     bool devInit = false, devOk = false;
     cudaStream_t stream = nullptr;
-    DevBuf arena, vout, prims, primsPh, pool, poolPh, binCount, bins, counters;
+    DevBuf arena, vout, prims, primsPh, pool, poolPh, binCount, bins;
+    PFDevCounters *counters = nullptr;      // on the device, in the last flush's staging copy
     DevBuf rowInfo, rowGroup;               // per item and per 32 items, their records' rows (BGRA8 targets)
     uint32_t cap = 256, poolCap = 4096;
     int rasterCtasPerSM = 0;                // 0: as many raster CTAs per SM as fit
@@ -1473,7 +1474,6 @@ bool device_init(Renderer *r)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&r->pinStream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->upDone, cudaEventDisableTiming);
     if (e != cudaSuccess) { report_device_failure("cudaStreamCreate", e); r->devStatus |= PF_DEVICE_NO_GPU; return false; }
-    if (!r->counters.ensure(sizeof(PFDevCounters))) { r->devStatus |= PF_DEVICE_ALLOC_FAIL; return false; }
     if (cudaMallocHost((void **)&r->hostCounters, sizeof(PFDevCounters)) != cudaSuccess) {
         cudaGetLastError(); r->devStatus |= PF_DEVICE_ALLOC_FAIL; return false;
     }
@@ -1486,7 +1486,7 @@ void release_renderer(Renderer *r)
     if (r->graph) { cudaGraphExecDestroy(r->graph); r->graph = nullptr; }
     if (r->devOk) {
         r->arena.release(); r->vout.release(); r->prims.release(); r->primsPh.release(); r->pool.release();
-        r->poolPh.release(); r->binCount.release(); r->bins.release(); r->counters.release();
+        r->poolPh.release(); r->binCount.release(); r->bins.release(); r->counters = nullptr;
         r->rowInfo.release(); r->rowGroup.release();
         if (r->hostCounters) cudaFreeHost(r->hostCounters);
         if (r->evStart) { cudaEventDestroy(r->evStart); cudaEventDestroy(r->evEnd); }
@@ -1645,15 +1645,17 @@ bool flush(Renderer *r)
 
     // --- framebuffers used: device copies ------------------------------------------
     std::vector<PFframebuffer *> used;
-    for (auto &cmd : cmds)
-        if (std::find(used.begin(), used.end(), cmd.fb) == used.end()) used.push_back(cmd.fb);
+    std::vector<int> firstCmd;                                     // the first command that touches it
+    std::unordered_map<const PFframebuffer *, size_t> slot;        // its place in used
+    for (size_t ci = 0; ci < cmds.size(); ci++)
+        if (slot.emplace(cmds[ci].fb, used.size()).second) { used.push_back(cmds[ci].fb); firstCmd.push_back((int)ci); }
     std::vector<FBMirror *> mirrors;
     for (PFframebuffer *fb : used) {
         FBMirror *m = mirror_for(r, fb);
         if (!m) return fail("cudaMalloc(framebuffer)", cudaErrorMemoryAllocation);
         mirrors.push_back(m);
     }
-    auto mirrorOf = [&](PFframebuffer *fb) { return mirrors[std::find(used.begin(), used.end(), fb) - used.begin()]; };
+    auto mirrorOf = [&](PFframebuffer *fb) { return mirrors[slot.at(fb)]; };
 
     // --- staging: states, segments, explicit items, targets join the block --------
     const size_t nStates = r->states.size(), nSegs = r->segs.size();
@@ -1662,6 +1664,17 @@ bool flush(Renderer *r)
     size_t nTargetsTotal = 0;
     for (auto &o : ops) if (o.kind == 0) nTargetsTotal += o.targets.size();
     int64_t targetsOff = r->staging.alloc(std::max<size_t>(nTargetsTotal, 1) * sizeof(PFTarget));
+    // the counters start from their staged values, and the pixels 0..7 that a
+    // leading fused pfClear keeps travel here too: each was a copy of its own,
+    // a launch and a switch between copy engine and kernels
+    const int64_t countersOff = r->staging.alloc(sizeof(PFDevCounters));
+    std::vector<int64_t> headOff(used.size(), -1);                 // 8 raw pixels, then 8 depths
+    for (auto &o : ops)
+        for (size_t k = 0; o.kind == 0 && k < o.targets.size(); k++) {
+            const size_t u = slot.at(o.targets[k]);
+            if (o.clearCmd[k] >= 0 && o.clearCmd[k] == firstCmd[u] && cmds[o.clearCmd[k]].kind == CMD_CLEAR)
+                headOff[u] = r->staging.alloc(8 * mirrors[u]->bpp + 8 * sizeof(float));
+        }
     for (auto &rec : r->segs) {
         if (!rec.records.empty()) {
             rec.recordsOff = r->staging.alloc(rec.records.size() * sizeof(PFVertexIn));
@@ -1761,6 +1774,17 @@ bool flush(Renderer *r)
                 const Cmd &cl = cmds[o.clearCmd[k]];
                 T.clearMode = (cl.kind == CMD_FILL) ? 2 : 1; T.clearDepth = cl.depth;
                 clear_raw(m->fmt, cl, T.clearRaw);
+                const size_t u = slot.at(o.targets[k]);
+                if (headOff[u] >= 0 && o.clearCmd[k] == firstCmd[u]) {
+                    // (the flush's only use of these bytes: the host's pixels as they are now)
+                    uint8_t *h = r->staging.base + headOff[u];
+                    std::memcpy(h, m->tex->pixels, 8 * m->bpp);
+                    T.headColor = (const uint32_t *)(dbase + headOff[u]);
+                    if (m->depthUserVisible || !m->depthOnDevice) {
+                        std::memcpy(h + 8 * m->bpp, m->hostDepth, 8 * sizeof(float));
+                        T.headDepth = (const float *)(dbase + headOff[u] + 8 * m->bpp);
+                    }
+                }
             }
         }
         L.segs = (const PFSegment *)(dbase + segsOff) + o.segBegin;
@@ -1774,6 +1798,10 @@ bool flush(Renderer *r)
         tgCursor += o.targets.size();
         maxVerts = std::max(maxVerts, v); maxItems = std::max(maxItems, it); maxTiles = std::max(maxTiles, tiles);
     }
+    PFDevCounters init{};
+    init.abortCommand = 0xffffffffu;
+    std::memcpy(r->staging.base + countersOff, &init, sizeof init);
+    PFDevCounters *dcnt = r->counters = (PFDevCounters *)(dbase + countersOff);
     cudaError_t e = cudaMemcpyAsync(dbase, r->staging.base, total, cudaMemcpyHostToDevice, st);
     settle_pinned(r);                               // (a flush inside a drawing call)
     if (e == cudaSuccess && r->upBytes) {            // the record-time uploads come first
@@ -1785,14 +1813,14 @@ bool flush(Renderer *r)
     // --- framebuffers: bring host content to the device unless the first
     //     operation touching a framebuffer overwrites it --------------------------
     for (size_t u = 0; u < used.size(); u++) {
-        PFframebuffer *fb = used[u];
         FBMirror *m = mirrors[u];
         const size_t n = m->w * m->h;
-        const Cmd *first = nullptr;
-        for (auto &cmd : cmds) if (cmd.fb == fb) { first = &cmd; break; }
+        const Cmd *first = &cmds[(size_t)firstCmd[u]];
         const bool uploadDepth = m->depthUserVisible || !m->depthOnDevice;
         if (first->kind == CMD_FILL) {
             // every pixel is overwritten first
+        } else if (headOff[u] >= 0) {
+            // cleared by the draw that follows: k_vertex puts pixels 0..7 in place
         } else if (first->kind == CMD_CLEAR) {
             // the clear leaves pixels 0..7 (and reads pixel 0 for the tail;
             // the packed 16-bit formats keep their tail, see k_clear)
@@ -1810,7 +1838,6 @@ bool flush(Renderer *r)
         m->depthOnDevice = true;
     }
 
-    PFDevCounters *dcnt = (PFDevCounters *)r->counters.p;
     uint32_t startOp = 0;
     r->lastOps.clear();
     for (void *q : r->splitMem) cudaFree(q);
@@ -1851,7 +1878,7 @@ bool flush(Renderer *r)
             acc += sg.nItems;
         }
         std::vector<PFTarget> TA = opTargets[oi], TB = opTargets[oi];
-        for (auto &t : TB) t.clearMode = 0;
+        for (auto &t : TB) { t.clearMode = 0; t.headColor = nullptr; t.headDepth = nullptr; }
         PFBatchLaunch LA = launches[oi], LB = launches[oi];
         auto place = [&](std::vector<PFSegment> &segs, std::vector<PFTarget> &tg, PFBatchLaunch &L) -> bool {
             uint32_t v = 0, it = 0;
@@ -1893,11 +1920,11 @@ bool flush(Renderer *r)
             r->devStatus |= PF_DEVICE_ALLOC_FAIL;
             return fail("cudaMalloc(scratch)", cudaErrorMemoryAllocation);
         }
-        PFDevCounters init{};
-        init.abortCommand = 0xffffffffu;
-        *r->hostCounters = init;
-        e = cudaMemcpyAsync(dcnt, r->hostCounters, sizeof(PFDevCounters), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return fail("cudaMemcpyAsync(counters)", e);
+        if (attempt) {
+            *r->hostCounters = init;
+            e = cudaMemcpyAsync(dcnt, r->hostCounters, sizeof(PFDevCounters), cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) return fail("cudaMemcpyAsync(counters)", e);
+        }
         size_t nRaster = 0;
         if (r->timing) {
             if (!r->evStart) { cudaEventCreate(&r->evStart); cudaEventCreate(&r->evEnd); }
@@ -2031,7 +2058,7 @@ float replay(Renderer *r, uint32_t n)
 {
     if (!r->devOk || r->lastOps.empty() || n == 0) return -1.0f;
     cudaStream_t st = r->stream;
-    PFDevCounters *dcnt = (PFDevCounters *)r->counters.p;
+    PFDevCounters *dcnt = r->counters;
     if (!r->graphValid) {
         if (r->graph) { cudaGraphExecDestroy(r->graph); r->graph = nullptr; }
         PFDevCounters init{};

@@ -28,6 +28,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <mutex>
 #include "pf_layout.h"
 #include "pf_device.h"
 #include "pf_pixfmt.h"
@@ -400,10 +401,12 @@ __device__ __forceinline__ int seg_of_item(const PFSegment *segs, int nSegs, uin
 }
 
 // One thread per vertex of the batch.  The grid also clears the tile bin
-// counters and the per-batch counters for k_items (so no memset launches).
+// counters and the per-batch counters for k_items (so no memset launches),
+// and puts the pixels that a fused clear keeps in place (a copy of their own
+// costs a small launch more than it moves).
 __global__ void k_vertex(const PFSegment *__restrict__ segs, int nSegs, const PFDrawState *__restrict__ states,
                          PFVertexOut *__restrict__ out, uint32_t nVerts, PFDevCounters *cnt,
-                         uint32_t *__restrict__ binCount, uint32_t nTiles)
+                         uint32_t *__restrict__ binCount, uint32_t nTiles, const PFTarget *__restrict__ targets, int nTargets)
 {
     __shared__ int sUniform, sAborted;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -428,6 +431,14 @@ __global__ void k_vertex(const PFSegment *__restrict__ segs, int nSegs, const PF
         cnt->clipCount = 0; cnt->batchRasterized = 0; cnt->tileQueue = 0; cnt->sortQueue = 0;
         cnt->tileListCount = 0;
         for (int l = 0; l < PF_HEAVY_LEVELS; l++) cnt->heavyCount[l] = 0;
+    }
+    if (g < (uint32_t)nTargets) {
+        // the pixels a fused pfClear keeps, which came with the draw states
+        const PFTarget &T = targets[g];
+        if (T.headColor)
+            for (int i = 0; i < 2 * pff_bytes(T.fmt); i++) static_cast<uint32_t *>(T.color)[i] = T.headColor[i];
+        if (T.headDepth)
+            for (int i = 0; i < 8; i++) T.depth[i] = T.headDepth[i];
     }
     if (g >= nVerts) return;
     // the segment and its draw state are read in place (one address for the
@@ -2639,7 +2650,8 @@ cudaError_t pfd_launch_vertex(const PFBatchLaunch &L, cudaStream_t st)
 {
     const uint32_t nTiles = L.totalTiles;
     const size_t work = L.nVerts > nTiles ? L.nVerts : nTiles;
-    k_vertex<<<grid_for(work, 128), 128, 0, st>>>(L.segs, L.nSegs, L.states, L.vout, L.nVerts, L.cnt, L.binCount, nTiles);
+    k_vertex<<<grid_for(work, 128), 128, 0, st>>>(L.segs, L.nSegs, L.states, L.vout, L.nVerts, L.cnt, L.binCount, nTiles,
+                                               L.targets, L.nTargets);
     return cudaGetLastError();
 }
 
@@ -2676,12 +2688,40 @@ static RasterArgs raster_args(const PFBatchLaunch &L)
                        L.targets, L.nTargets, L.totalTiles, L.cnt, L.command, L.anyPhong };
 }
 
+// CTAs of `kernel` that fit on an SM, its shared-memory limits set.  Asked of
+// the driver once per device, kernel and size: the three calls for every
+// launch of a frame take about as long as a small frame's kernel.
+static cudaError_t ctas_per_sm(const void *kernel, int block, size_t smem, bool maxShared, int &fit)
+{
+    struct Known { const void *kernel; int dev, block, fit; size_t smem; };
+    static std::mutex m;
+    static Known known[64];
+    static int count = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(m);
+    size_t limit = 0;                                  // what the kernel's limit was raised to
+    for (int i = 0; i < count; i++) {
+        const Known &k = known[i];
+        if (k.kernel != kernel || k.dev != dev) continue;
+        if (k.block == block && k.smem == smem) { fit = k.fit; return cudaSuccess; }
+        limit = k.smem > limit ? k.smem : limit;
+    }
+    if (smem > limit) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && maxShared)                 // the CTAs' shared memory, not L1, bounds how many fit on an SM
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, block, smem);
+    if (e == cudaSuccess && count < 64) known[count++] = Known{ kernel, dev, block, fit, smem };
+    return e;
+}
+
 // Persistent grid of `kernel`: as many CTAs as fit on the GPU at once, at
 // most `perSM` per SM (0: as many as fit), at most `units`.
-static cudaError_t persistent_grid(const void *kernel, int block, size_t smem, int perSM, uint32_t units, uint32_t &grid)
+static cudaError_t persistent_grid(const void *kernel, int block, size_t smem, bool maxShared, int perSM, uint32_t units, uint32_t &grid)
 {
     int fit = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, block, smem);
+    cudaError_t e = ctas_per_sm(kernel, block, smem, maxShared, fit);
     if (e != cudaSuccess) return e;
     uint32_t per = (uint32_t)(fit > 0 ? fit : 1);
     if (perSM > 0) per = min(per, (uint32_t)perSM);
@@ -2694,9 +2734,8 @@ cudaError_t pfd_launch_binsort(const PFBatchLaunch &L, cudaStream_t st)
     if (L.totalTiles == 0) return cudaSuccess;
     uint32_t N = 32; while (N < L.cap) N <<= 1;
     const size_t smem = 2 * (size_t)N * sizeof(uint32_t);             // merge source and target
-    cudaError_t e = cudaFuncSetAttribute(k_binsort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     uint32_t grid = 0;
-    if (e == cudaSuccess) e = persistent_grid((const void *)k_binsort, SORT_THREADS, smem, 0, L.totalTiles, grid);
+    cudaError_t e = persistent_grid((const void *)k_binsort, SORT_THREADS, smem, false, 0, L.totalTiles, grid);
     if (e != cudaSuccess) return e;
     return launch_serialized(k_binsort, grid, SORT_THREADS, smem, st, raster_args(L));
 }
@@ -2714,21 +2753,19 @@ cudaError_t pfd_launch_raster(const PFBatchLaunch &L, cudaStream_t st)
     void (*kernel)(RasterArgs) =
         L.generic ? (L.anyPhong ? raster_kernel<true, true>(warps) : raster_kernel<true, false>(warps))
                   : (L.anyPhong ? raster_kernel<false, true>(warps) : raster_kernel<false, false>(warps));
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)     // the CTAs' shared memory, not L1, bounds how many fit on an SM
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     uint32_t grid = 0;
-    if (e == cudaSuccess) e = persistent_grid((const void *)kernel, warps * 32, smem, L.rasterCtasPerSM,
-                                              (2u * L.totalTiles + (uint32_t)warps - 1) / (uint32_t)warps, grid);  // half tiles
+    cudaError_t e = persistent_grid((const void *)kernel, warps * 32, smem, true, L.rasterCtasPerSM,
+                                    (2u * L.totalTiles + (uint32_t)warps - 1) / (uint32_t)warps, grid);       // half tiles
     if (e != cudaSuccess) return e;
     e = launch_serialized(kernel, grid, (unsigned)(warps * 32), smem, st, raster_args(L));
     if (e != cudaSuccess || L.rowCount == 0 || !L.rowInfo || !L.rowGroup) return e;
     const bool inSmem = L.rowMaxW <= ROW_SMEM_MAX_W;
-    const uint32_t rowW = (L.rowMaxW + 3u) & ~3u;
+    const uint32_t rowW = (L.rowMaxW + 255u) & ~255u;                                   // (few sizes: ctas_per_sm keeps them)
     const size_t rsm = sizeof(RowShared) + (inSmem ? (size_t)rowW * 8 : 0);            // colour and depth of the row
     auto rows = inSmem ? (L.anyPhong ? k_rows<true, true> : k_rows<true, false>)
                        : (L.anyPhong ? k_rows<false, true> : k_rows<false, false>);
-    e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
+    int fit = 0;
+    e = ctas_per_sm((const void *)rows, ROW_THREADS, rsm, false, fit);
     if (e != cudaSuccess) return e;
     return launch_serialized(rows, L.rowCount, ROW_THREADS, rsm, st, raster_args(L), L.segs, L.nSegs,
                              (const uint64_t *)L.rowInfo, (const uint64_t *)L.rowGroup, rowW);

@@ -125,7 +125,9 @@ typedef struct {
     uint32_t clearRaw[4];         /* the clear colour as stored: SIMD setter (pfClear), scalar (fill) */
     float clearDepth;
     uint32_t fmt;                 /* PFF_* framebuffer format */
-} PFTarget;                       /* 64 bytes */
+    const uint32_t *headColor;    /* clearMode 1: the framebuffer's pixels 0..7 as the host holds them, which */
+    const float *headDepth;       /* k_vertex puts in place (NULL: the device's are current) */
+} PFTarget;                       /* 80 bytes */
 
 /* Transformed vertex. */
 typedef struct PF_ALIGN16 {

@@ -135,11 +135,16 @@ extern "C" int pfgbDrawTrianglesStatic(const float *positions, const uint32_t *c
     T.tilesX = (width + PF_TILE - 1) / PF_TILE; T.tilesY = (height + PF_TILE - 1) / PF_TILE;
     T.tileBase = 0; T.clearMode = 0;
 
-    // pageable sources: these copies return once the data left the stack
-    cudaError_t e = cudaMemcpyAsync(s + kOffState, &S, sizeof S, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s + kOffSeg, &G, sizeof G, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s + kOffCnt, &C, sizeof C, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s + kOffTarget, &T, sizeof T, cudaMemcpyHostToDevice, st);
+    // the four lie one after the other in the scratch: one copy, from
+    // pageable memory (it returns once the data left the stack)
+    static_assert(kOffState == 0 && kOffVout <= 4096, "the head of the scratch is small");
+    unsigned char head[kOffTarget + sizeof T];
+    std::memset(head, 0, sizeof head);
+    std::memcpy(head + kOffState, &S, sizeof S);
+    std::memcpy(head + kOffSeg, &G, sizeof G);
+    std::memcpy(head + kOffCnt, &C, sizeof C);
+    std::memcpy(head + kOffTarget, &T, sizeof T);
+    cudaError_t e = cudaMemcpyAsync(s, head, sizeof head, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) { cudaGetLastError(); return PFGB_STATIC_E_CUDA; }
 
     PFBatchLaunch L{};
