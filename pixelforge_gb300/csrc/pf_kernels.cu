@@ -924,9 +924,9 @@ __device__ __forceinline__ uint64_t row_group(uint64_t w)
     return __any_sync(0xffffffffu, any) ? (1ull | (uint64_t)lo << 16 | (uint64_t)hi << 40) : 0ull;
 }
 
-// rowInfo[g] of an item whose only record is P (kept) or that has none;
-// out of line, so that the set-up path keeps its registers
-__device__ __noinline__ void store_row_info(uint64_t *rowInfo, uint32_t g, const PFPrim &P, bool kept)
+// rowInfo[g] of an item whose only record is P (kept) or that has none.
+// (In line: taking the record's address would keep it in local memory.)
+__device__ __forceinline__ void store_row_info(uint64_t *rowInfo, uint32_t g, const PFPrim &P, bool kept)
 {
     uint64_t rows = 0;
     if (kept) row_info_add(rows, 0, P);
@@ -1043,9 +1043,10 @@ __device__ __forceinline__ bool item_setup(const PFSegment &sg, const PFDrawStat
     }
     SVert s[3];
     for (int m = 0; m < 3; m++) {
-        const PFVertexOut &o = *V[m];
-        const float4 h = hv[m];
-        const float2 uv = *reinterpret_cast<const float2 *>(o.uv);
+        // (the vertex's other three 16-byte words: uv and colours, normal and
+        // position)
+        const float4 *vw = reinterpret_cast<const float4 *>(V[m]);
+        const float4 h = hv[m], uv = vw[1];
         if (is2D) {
             to_screen(S, h.x, h.y, s[m].sx, s[m].sy);
             s[m].z = h.z; s[m].u = uv.x; s[m].v = uv.y;
@@ -1056,9 +1057,13 @@ __device__ __forceinline__ bool item_setup(const PFSegment &sg, const PFDrawStat
             to_screen(S, h.x * invW, h.y * invW, s[m].sx, s[m].sy);
             s[m].z = hz;
         }
-        s[m].c = o.col[face];
-        if (S.flags & PFS_PHONG)
-            for (int i = 0; i < 3; i++) { s[m].n[i] = o.n[i]; s[m].p[i] = o.p[i]; }
+        s[m].c = __float_as_uint(face ? uv.w : uv.z);
+        if (S.flags & PFS_PHONG) {
+            const float4 np = vw[2];
+            const float2 pp = *reinterpret_cast<const float2 *>(vw + 3);
+            s[m].n[0] = np.x; s[m].n[1] = np.y; s[m].n[2] = np.z;
+            s[m].p[0] = np.w; s[m].p[1] = pp.x; s[m].p[2] = pp.y;
+        }
     }
     const bool kept = setup_prim(S, face, !is2D, s[0], s[1], s[2], sg.state, P);
     if (O.rowInfo) store_row_info(O.rowInfo, g, P, kept);
