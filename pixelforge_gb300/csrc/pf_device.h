@@ -26,6 +26,7 @@ struct PFBatchLaunch {
     PFVertexOut *vout;
     uint32_t nVerts;
     uint32_t nItems;
+    uint32_t itemSpan;        /* most items between the first and the last of one target's, inclusive (k_binsort) */
     PFPrim *prims;            /* nItems records (sub-triangle 0 of each item) */
     PFPrimPhong *primsPh;
     PFPrim *pool;             /* clipped sub-triangles >= 1 */

@@ -1750,12 +1750,16 @@ bool flush(Renderer *r)
             o.clearCmd.swap(cl);
         }
         uint32_t v = 0, it = 0, tiles = 0;
+        std::vector<uint32_t> firstItem(o.targets.size(), 0xffffffffu);
         for (int si = o.segBegin; si < o.segEnd; si++) {
             hseg[si].vtxBase = v; hseg[si].itemBase = it;
             v += hseg[si].nVerts; it += hseg[si].nItems;
             PFframebuffer *fb = r->segs[si].fb;
             hseg[si].target = (int32_t)(std::find(o.targets.begin(), o.targets.end(), fb) - o.targets.begin());
             if (hs[hseg[si].state].flags & PFS_PHONG) anyPhong = true;
+            uint32_t &first = firstItem[(size_t)hseg[si].target];
+            first = std::min(first, hseg[si].itemBase);
+            L.itemSpan = std::max(L.itemSpan, it - first);
         }
         for (size_t k = 0; k < o.targets.size(); k++) {
             FBMirror *m = mirrorOf(o.targets[k]);

@@ -150,7 +150,7 @@ extern "C" int pfgbDrawTrianglesStatic(const float *positions, const uint32_t *c
     PFBatchLaunch L{};
     L.segs = (const PFSegment *)(s + kOffSeg); L.nSegs = 1;
     L.states = (const PFDrawState *)(s + kOffState);
-    L.vout = (PFVertexOut *)(s + kOffVout); L.nVerts = G.nVerts; L.nItems = G.nItems;
+    L.vout = (PFVertexOut *)(s + kOffVout); L.nVerts = G.nVerts; L.nItems = L.itemSpan = G.nItems;
     L.prims = (PFPrim *)(s + kOffPrims); L.primsPh = (PFPrimPhong *)(s + kOffPh);
     L.pool = (PFPrim *)(s + kOffPool); L.poolPh = (PFPrimPhong *)(s + kOffPh); L.poolCap = kPoolCap;
     L.binCount = (uint32_t *)(s + kOffBinCount); L.bins = (uint32_t *)(s + kOffBins); L.cap = kBinCap;
