@@ -833,7 +833,7 @@ __device__ __forceinline__ void item_vertices(const PFSegment &sg, uint32_t k, u
             j = sg.nVerts - 1;                         // device indices (pfDrawElementsDevice): clamped, flagged
             atomicOr(status, (unsigned)PFD_BOUNDS);
         }
-        v[m] = sg.vtxBase + j;
+        v[m] = sg.vtxRead + j;
     }
 }
 

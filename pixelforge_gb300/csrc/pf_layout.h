@@ -87,7 +87,9 @@ enum { PF_ITEMS_TRIS = 0, PF_ITEMS_EXPLICIT = 1 };
 typedef struct {
     int32_t state;
     int32_t srcKind;
-    uint32_t vtxBase;             /* first transformed vertex of this segment */
+    uint32_t vtxBase;             /* first transformed vertex of this segment, as k_vertex numbers them */
+    uint32_t vtxRead;             /* first transformed vertex its items read: vtxBase, or an earlier segment's
+                                     that transforms the same vertices the same way (k_vertex skips this one) */
     uint32_t nVerts;
     uint32_t itemBase;            /* first item (global order number in the batch) */
     uint32_t nItems;
@@ -111,7 +113,7 @@ typedef struct {
     uint32_t itemSkip;            /* items of the draw before this segment's first (a draw split into passes) */
     const void *prebuilt;         /* PFPrim records of points and lines set up on the host: an explicit
                                      item {i, 0, 0, -1} stands for record i */
-} PFSegment;                      /* 144 bytes */
+} PFSegment;                      /* 152 bytes */
 
 /* A framebuffer rendered by a batch.  Its tiles are numbered
  * tileBase .. tileBase + tilesX*tilesY - 1 in the batch's bin arrays. */
