@@ -2602,54 +2602,81 @@ __global__ void k_fill(void *color, uint32_t fmt, float *depth, size_t n, uint4 
 }
 
 // Post-process hooks (pfPostProcess, context.c:2397-2441) and pfFogProcess
-// (context.c:2288-2351), through the scalar getter and setter.  The hooks
-// rewrite every pixel; the fog writes only the pixels past its start.
+// (context.c:2288-2351) on the colour c of pixel i, as the scalar getter
+// reads it.  The hooks rewrite every pixel; the fog writes only the pixels
+// past its start (false: keep the pixel).
+__device__ __forceinline__ bool hook_pixel(uint32_t &c, float depth, size_t i, int hook, const PFHookParams &hp)
+{
+    bool write = true;
+    if (hook == 1) {          // linear fog on depth
+        float d = (depth + hp.znear) / (hp.zfar + hp.znear);
+        float f = (hp.end - d) / (hp.end - hp.start);
+        f = x86_min(x86_max(f, 0.0f), 1.0f);
+        uint32_t k = (uint32_t)x86_cvt_trunc(f * 255.0f);
+        uint32_t r = 0;
+        for (int ch = 0; ch < 4; ch++) r |= (((chn(c, ch) * k + chn(hp.color, ch) * (255u - k)) / 255u) & 255u) << (8 * ch);
+        c = r;
+    } else if (hook == 3) {   // pfFogProcess (context.c:2288-2351)
+        const float d = depth;
+        write = d > hp.start;
+        const uint32_t alpha = hp.color >> 24, fc = hp.color & 0x00ffffffu;
+        if (d >= hp.end) {
+            const uint32_t f = fc | (alpha << 24);
+            c = alpha == 255u ? f : blend_sisd(1, f, c);
+        } else if (d > hp.start) {
+            float t = 0.0f;
+            const float invLen = __frcp_rn(hp.end - hp.start);
+            if (hp.mode == 0) t = (d - hp.start) * invLen;
+            else if (hp.mode == 1) t = 1.0f - (float)exp((double)(-hp.density * (d - hp.start)));
+            else if (hp.mode == 2) t = 1.0f - (float)exp2((double)(-hp.density * (d - hp.start)));
+            const uint32_t a = (uint32_t)x86_cvt_trunc(t * (float)alpha) & 255u;
+            c = blend_sisd(1, fc | (a << 24), c);
+        }
+    } else if (hook == 2) {   // grayscale
+        uint32_t gy = (77u * chn(c, 0) + 150u * chn(c, 1) + 29u * chn(c, 2)) >> 8;
+        c = gy | (gy << 8) | (gy << 16) | (c & 0xff000000u);
+    } else if (hook == 4) {   // ordered 3x3 dither (examples/raylib/raylib_PostProcess.c:7-19)
+        const uint32_t x = (uint32_t)(i % hp.width), y = (uint32_t)(i / hp.width);
+        // the matrix {{230, 51, 128}, {25, 102, 179}, {154, 205, 77}}, row
+        // x % 3, column y % 3: its first eight bytes packed low to high
+        const uint32_t m = x % 3u * 3u + y % 3u;
+        const uint32_t dv = m < 8u ? (uint32_t)((0xCD9AB366198033E6ull >> (8u * m)) & 255u) : 77u;
+        const uint32_t avg = (chn(c, 0) + chn(c, 1) + chn(c, 2)) / 3u;
+        c = (avg >= dv) ? 0xffffffffu : 0u;
+    }
+    return write;
+}
+
+// RGBA / unsigned byte (whose scalar getter and setter are the identity):
+// four pixels a thread in 16-byte accesses, a thread's loads all under way at
+// once.  Bound by its loads' latency: one pixel a thread and step, 20 us for
+// the 1080p linear fog, now 8.7 (24.9 MB read and written).
 __global__ void k_hook(void *color, uint32_t fmt, const float *depth, size_t n, int hook, PFHookParams hp,
                        const PFDevCounters *cnt, uint32_t command)
 {
     if (cnt->abortCommand <= command) return;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    size_t done = 0;
+    if (fmt == PFF_RGBA8 && (((uintptr_t)color | (uintptr_t)depth) & 15u) == 0) {
+        const size_t n4 = n / 4;
+        for (size_t q = first; q < n4; q += stride) {
+            uint4 v = reinterpret_cast<const uint4 *>(color)[q];
+            const float4 z = reinterpret_cast<const float4 *>(depth)[q];
+            // (a pixel the hook leaves is stored as it was read)
+            const uint4 o = v;
+            if (!hook_pixel(v.x, z.x, 4 * q, hook, hp)) v.x = o.x;
+            if (!hook_pixel(v.y, z.y, 4 * q + 1, hook, hp)) v.y = o.y;
+            if (!hook_pixel(v.z, z.z, 4 * q + 2, hook, hp)) v.z = o.z;
+            if (!hook_pixel(v.w, z.w, 4 * q + 3, hook, hp)) v.w = o.w;
+            reinterpret_cast<uint4 *>(color)[q] = v;
+        }
+        done = 4 * n4;
+    }
+    for (size_t i = done + first; i < n; i += stride) {
         uint32_t raw[4];
         pff_load(fmt, color, i, raw);
         uint32_t c = pff_get_sisd(fmt, raw);
-        bool write = true;
-        if (hook == 1) {          // linear fog on depth
-            float d = (depth[i] + hp.znear) / (hp.zfar + hp.znear);
-            float f = (hp.end - d) / (hp.end - hp.start);
-            f = x86_min(x86_max(f, 0.0f), 1.0f);
-            uint32_t k = (uint32_t)x86_cvt_trunc(f * 255.0f);
-            uint32_t r = 0;
-            for (int ch = 0; ch < 4; ch++) r |= (((chn(c, ch) * k + chn(hp.color, ch) * (255u - k)) / 255u) & 255u) << (8 * ch);
-            c = r;
-        } else if (hook == 3) {   // pfFogProcess (context.c:2288-2351)
-            const float d = depth[i];
-            write = d > hp.start;
-            const uint32_t alpha = hp.color >> 24, fc = hp.color & 0x00ffffffu;
-            if (d >= hp.end) {
-                const uint32_t f = fc | (alpha << 24);
-                c = alpha == 255u ? f : blend_sisd(1, f, c);
-            } else if (d > hp.start) {
-                float t = 0.0f;
-                const float invLen = __frcp_rn(hp.end - hp.start);
-                if (hp.mode == 0) t = (d - hp.start) * invLen;
-                else if (hp.mode == 1) t = 1.0f - (float)exp((double)(-hp.density * (d - hp.start)));
-                else if (hp.mode == 2) t = 1.0f - (float)exp2((double)(-hp.density * (d - hp.start)));
-                const uint32_t a = (uint32_t)x86_cvt_trunc(t * (float)alpha) & 255u;
-                c = blend_sisd(1, fc | (a << 24), c);
-            }
-        } else if (hook == 2) {   // grayscale
-            uint32_t gy = (77u * chn(c, 0) + 150u * chn(c, 1) + 29u * chn(c, 2)) >> 8;
-            c = gy | (gy << 8) | (gy << 16) | (c & 0xff000000u);
-        } else if (hook == 4) {   // ordered 3x3 dither (examples/raylib/raylib_PostProcess.c:7-19)
-            const uint32_t x = (uint32_t)(i % hp.width), y = (uint32_t)(i / hp.width);
-            // the matrix {{230, 51, 128}, {25, 102, 179}, {154, 205, 77}}, row
-            // x % 3, column y % 3: its first eight bytes packed low to high
-            const uint32_t m = x % 3u * 3u + y % 3u;
-            const uint32_t dv = m < 8u ? (uint32_t)((0xCD9AB366198033E6ull >> (8u * m)) & 255u) : 77u;
-            const uint32_t avg = (chn(c, 0) + chn(c, 1) + chn(c, 2)) / 3u;
-            c = (avg >= dv) ? 0xffffffffu : 0u;
-        }
-        if (write) {
+        if (hook_pixel(c, depth[i], i, hook, hp)) {
             pff_set_sisd(fmt, c, raw);
             pff_store(fmt, color, i, raw);
         }
@@ -2868,9 +2895,9 @@ cudaError_t pfd_launch_clear(void *color, uint32_t fmt, float *depth, size_t n, 
 cudaError_t pfd_launch_hook(void *color, uint32_t fmt, const float *depth, size_t n, int hook, const PFHookParams &hp,
                             const PFDevCounters *cnt, uint32_t command, cudaStream_t st)
 {
-    unsigned grid = (unsigned)min((size_t)152 * 8, (n + 255) / 256);
-    if (grid == 0) return cudaSuccess;
-    k_hook<<<grid, 256, 0, st>>>(color, fmt, depth, n, hook, hp, cnt, command);
+    unsigned grid = (unsigned)min((size_t)pfd_sm_count() * 16, (n / 4 + 127) / 128 + 1);
+    if (n == 0) return cudaSuccess;
+    k_hook<<<grid, 128, 0, st>>>(color, fmt, depth, n, hook, hp, cnt, command);
     return cudaGetLastError();
 }
 
