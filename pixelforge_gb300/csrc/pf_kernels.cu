@@ -1683,12 +1683,14 @@ __device__ __forceinline__ void tile_list(unsigned long long m, uint32_t off, ui
 }
 
 // GEN: a target is not RGBA / unsigned byte.  PHONG: a draw state lights per
-// fragment; without that code the 80 registers hold everything (with it 52
-// bytes a thread spill): sphere1080 58 -> 56 us, 64-soup batch 1,925 ->
-// 1,780.  Bound by instruction issue and the round trips of claims, bin keys
-// and records.
+// fragment; without that code nothing spills: sphere1080 58 -> 56 us,
+// 64-soup batch 1,925 -> 1,780.  Warps an SM, by what fits without spills:
+// 28 (72 registers; 24: 64-soup batch 1,555 -> 1,455, 8,192 small triangles
+// 32 -> 28; 32 warps: 1,505), GEN 24 (28: 35 -> 36.5 on RGBA half), PHONG 20
+// (24: phong1080 340 -> 312; 16: 362).  Bound by instruction issue and the
+// round trips of claims, bin keys and records.
 template <bool GEN, int WARPS, bool PHONG>
-__global__ void __launch_bounds__(WARPS * 32, 24 / WARPS) k_raster(RasterArgs a)
+__global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WARPS) k_raster(RasterArgs a)
 {
     extern __shared__ __align__(16) unsigned char rsmem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
