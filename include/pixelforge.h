@@ -515,7 +515,7 @@ PF_API PFfloat   pfgbReplay(PFuint n);
 #define PFGB_STATIC_MAX_HEIGHT      512
 #define PFGB_STATIC_BIN_CAPACITY    512       /* sub-triangles per 8x8 tile */
 #define PFGB_STATIC_CLIP_CAPACITY   32768     /* extra sub-triangles of clipped triangles */
-#define PFGB_STATIC_SCRATCH_BYTES   16353024  /* 15.6 MiB */
+#define PFGB_STATIC_SCRATCH_BYTES   16615168  /* 15.8 MiB */
 #define PFGB_STATIC_E_TOO_LARGE     (-1)      /* more triangles or pixels than the limits */
 #define PFGB_STATIC_E_INVALID       (-2)      /* null pointer or invalid mode */
 #define PFGB_STATIC_E_CUDA          (-3)      /* a CUDA call failed */

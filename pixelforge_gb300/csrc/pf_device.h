@@ -29,6 +29,7 @@ struct PFBatchLaunch {
     uint32_t itemSpan;        /* most items between the first and the last of one target's, inclusive (k_binsort) */
     PFPrim *prims;            /* nItems records (sub-triangle 0 of each item) */
     PFPrimPhong *primsPh;
+    float4 *planes;           /* nItems depth planes of the records (depth_plane) */
     PFPrim *pool;             /* clipped sub-triangles >= 1 */
     PFPrimPhong *poolPh;
     uint32_t poolCap;

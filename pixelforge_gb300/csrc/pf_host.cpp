@@ -295,7 +295,7 @@ struct Renderer {
     // device
     bool devInit = false, devOk = false;
     cudaStream_t stream = nullptr;
-    DevBuf arena, vout, prims, primsPh, pool, poolPh, binCount, bins;
+    DevBuf arena, vout, prims, primsPh, planes, pool, poolPh, binCount, bins;
     PFDevCounters *counters = nullptr;      // on the device, in the last flush's staging copy
     DevBuf rowInfo, rowGroup;               // per item and per 32 items, their records' rows (BGRA8 targets)
     uint32_t cap = 256, poolCap = 4096;
@@ -1485,7 +1485,7 @@ void release_renderer(Renderer *r)
 {
     if (r->graph) { cudaGraphExecDestroy(r->graph); r->graph = nullptr; }
     if (r->devOk) {
-        r->arena.release(); r->vout.release(); r->prims.release(); r->primsPh.release(); r->pool.release();
+        r->arena.release(); r->vout.release(); r->prims.release(); r->primsPh.release(); r->planes.release(); r->pool.release();
         r->poolPh.release(); r->binCount.release(); r->bins.release(); r->counters = nullptr;
         r->rowInfo.release(); r->rowGroup.release();
         if (r->hostCounters) cudaFreeHost(r->hostCounters);
@@ -1945,6 +1945,7 @@ bool flush(Renderer *r)
         if (!r->vout.ensure((size_t)maxVerts * sizeof(PFVertexOut) + 64) ||
             !r->prims.ensure((size_t)maxItems * sizeof(PFPrim) + 128) ||
             !r->primsPh.ensure(anyPhong ? (size_t)maxItems * sizeof(PFPrimPhong) + 128 : 128) ||
+            !r->planes.ensure((size_t)maxItems * sizeof(float4)) ||
             !r->pool.ensure((size_t)r->poolCap * sizeof(PFPrim)) ||
             !r->poolPh.ensure(anyPhong ? (size_t)r->poolCap * sizeof(PFPrimPhong) : 128) ||
             !r->binCount.ensure((size_t)(((size_t)maxTiles + 31) & ~(size_t)31) * 4 * (2 + PF_HEAVY_LEVELS)) ||   // bin counters, tile lists
@@ -1983,6 +1984,7 @@ bool flush(Renderer *r)
                 PFBatchLaunch L = launches[oi];
                 L.vout = (PFVertexOut *)r->vout.p;
                 L.prims = (PFPrim *)r->prims.p; L.primsPh = (PFPrimPhong *)r->primsPh.p;
+                L.planes = (float4 *)r->planes.p;
                 L.pool = (PFPrim *)r->pool.p; L.poolPh = (PFPrimPhong *)r->poolPh.p; L.poolCap = r->poolCap;
                 L.binCount = (uint32_t *)r->binCount.p; L.bins = (uint32_t *)r->bins.p; L.cap = r->cap;
                 L.listStride = (uint32_t)(((size_t)maxTiles + 31) & ~(size_t)31);

@@ -5,13 +5,15 @@
 //   k_items    one thread per triangle-face item, in submission order:
 //              2D/3D decision, projection, polygon clipping of the rare items
 //              that cross a plane (triangles.c:157-280), setup, cull and
-//              order-keyed binning into 16x16 tiles (triangles.c:287-339)
-//   k_raster   one CTA per tile: restores submission order of the tile's
-//              bin, then per chunk of sub-triangles computes coverage with
+//              order-keyed binning into 8x8 tiles (triangles.c:287-339)
+//   k_binsort  long bins back into submission order
+//   k_raster   one warp per tile: restores submission order of a short
+//              bin, then per batch of sub-triangles computes coverage with
 //              the reference's integer edge functions, shades fragments
 //              densely and resolves each pixel's fragments in order (depth
 //              test, blend) (triangles.c:398-557); optionally starts from
 //              a fused clear
+//   k_rows     BGRA / unsigned-byte targets, one CTA per framebuffer row
 //   k_clear, k_fill, k_hook  framebuffer-wide passes (pfClear,
 //              pfClearFramebuffer, device post-process hooks)
 //
@@ -428,7 +430,7 @@ __global__ void k_vertex(const PFSegment *__restrict__ segs, int nSegs, const PF
     if (sAborted) return;
     for (uint32_t t = g; t < nTiles; t += gridDim.x * blockDim.x) binCount[t] = 0;
     if (g == 0) {
-        cnt->clipCount = 0; cnt->batchRasterized = 0; cnt->tileQueue = 0; cnt->sortQueue = 0;
+        cnt->clipCount = 0; cnt->batchRasterized = 0; cnt->batchFragments = 0; cnt->tileQueue = 0; cnt->sortQueue = 0;
         cnt->tileListCount = 0;
         for (int l = 0; l < PF_HEAVY_LEVELS; l++) cnt->heavyCount[l] = 0;
     }
@@ -507,17 +509,20 @@ struct BinArgs {
     const PFTarget *targets;
     PFDevCounters *cnt;
     uint32_t command;
+    float4 *planes;            // depth_plane of each item's sub-triangle 0
+    bool countSmall;           // triangles within 32x32 pixels are counted by k_items too
 };
 
 // Framebuffer geometry a sub-triangle is binned against.
 struct TileSpace {
     uint32_t W, H, tilesX, tileBase;
+    bool rows;                 // rasterized by k_rows, which counts its fragments
 };
 
 __device__ __forceinline__ TileSpace tile_space(const BinArgs &B, int target)
 {
     const PFTarget &t = B.targets[target];
-    return TileSpace{ t.W, t.H, t.tilesX, t.tileBase };
+    return TileSpace{ t.W, t.H, t.tilesX, t.tileBase, t.fmt == PFF_BGRA8 };
 }
 
 
@@ -548,14 +553,18 @@ struct EdgeTest {
     int32_t xMin, xMax, yMin, yMax;
     bool on;
 };
-__device__ __forceinline__ EdgeTest edge_test(const PFPrim &P, uint32_t W, uint32_t H)
+__device__ __forceinline__ bool edge_on(const PFPrim &P, uint32_t W, uint32_t H)
 {
-    EdgeTest E;
     const int32_t L = 1 << 13;
     const int32_t v[6] = { P.x1, P.y1, P.x2, P.y2, P.x3, P.y3 };
     bool ok = !(P.flags & PFP_KIND) && W <= (uint32_t)L && H <= (uint32_t)L &&
               P.xMin > -L && P.xMin < L && P.xMax > -L && P.xMax < L && P.yMin > -L && P.yMin < L && P.yMax > -L && P.yMax < L;
     for (int k = 0; k < 6; k++) ok = ok && v[k] > -L && v[k] < L;
+    return ok;
+}
+__device__ __forceinline__ EdgeTest edge_test(const PFPrim &P, bool ok)
+{
+    EdgeTest E;
     const int32_t vx[3] = { P.x2, P.x3, P.x1 }, vy[3] = { P.y2, P.y3, P.y1 };
     const int32_t sgn = (P.flags & 1u) ? -1 : 1;
     const int32_t sx[3] = { P.y3 - P.y2, P.y1 - P.y3, P.y2 - P.y1 }, sy[3] = { P.x2 - P.x3, P.x3 - P.x1, P.x1 - P.x2 };
@@ -645,13 +654,39 @@ __device__ __forceinline__ void list_tiles_warp(const BinArgs &B, uint32_t t, ui
     }
 }
 
+// Whether the record may raise a pixel's depth (a batch without such
+// records only lowers depths).
+__device__ __forceinline__ bool raises_depth(uint32_t rstate)
+{
+    const uint32_t func = (rstate >> 16) & 255u;
+    return (rstate & PFS_DEPTH_MASK) && !((rstate & PFS_DEPTH_TEST) && (func == 2u || func == 3u || func == 0u));
+}
+
+// What k_raster needs to know of a record to drop it before loading it: a
+// bound on its interpolated term 1 / depth over the image, the plane
+// x + y px + z py, and a bound w over the whole triangle.  The plane only
+// for triangles of more than a tile, whose corners' depths say little about
+// their depth in one tile; m bounds the sum of its absolute terms over the
+// tiles of the box, and 4e-6 m the rounding of this
+// evaluation, k_raster's and a covered fragment's own (some twenty
+// operations of 2^-24 each).  Infinite where there is no bound, w NaN when
+// the record may raise a depth.
+__device__ __forceinline__ float depth_bound(const PFPrim &P)
+{
+    const float inf = __int_as_float(0x7f800000);
+    if (raises_depth(P.rstate)) return __int_as_float(0x7fffffff);
+    if (!(P.zReject == P.zReject)) return inf;         // (none unless lo > 0 or hi < 0)
+    const float lo = fminf(P.z1, fminf(P.z2, P.z3)), hi = fmaxf(P.z1, fmaxf(P.z2, P.z3));
+    return hi * (lo > 0.0f ? 1.00001f : 0.99999f);
+}
+
 // Append `key` to the bin of every tile the sub-triangle touches (one
 // thread; used by the clipping path).
 __device__ void bin_prim(const BinArgs &B, const TileSpace &T, const PFPrim &P, uint32_t key)
 {
     uint32_t tx0, ty0, ntx, nty;
     if (!tile_range(T, P, tx0, ty0, ntx, nty)) return;
-    const EdgeTest ET = edge_test(P, T.W, T.H);
+    const EdgeTest ET = edge_test(P, edge_on(P, T.W, T.H));
     for (uint32_t ty = ty0; ty < ty0 + nty; ty++)
         for (uint32_t tx = tx0; tx < tx0 + ntx; tx++) {
             if (!tile_touched(ET, tx, ty, T.W, T.H)) continue;
@@ -660,6 +695,14 @@ __device__ void bin_prim(const BinArgs &B, const TileSpace &T, const PFPrim &P, 
             list_tile(B, t, slot, 1u);
             bin_slot(B, t, slot, key);
         }
+}
+
+// Whether the record's box is that of its vertices, inside the framebuffer.
+__device__ __forceinline__ bool whole_box(const PFPrim &P, const TileSpace &T)
+{
+    return P.xMin == min(P.x1, min(P.x2, P.x3)) && P.xMax == max(P.x1, max(P.x2, P.x3)) &&
+           P.yMin == min(P.y1, min(P.y2, P.y3)) && P.yMax == max(P.y1, max(P.y2, P.y3)) &&
+           P.xMin >= 0 && P.yMin >= 0 && (uint32_t)P.xMax <= T.W && (uint32_t)P.yMax < T.H;
 }
 
 // A lane's sub-triangle as its warp bins it, in shared memory: seven 16-byte
@@ -671,10 +714,14 @@ struct __align__(16) BinRec {
     int32_t x0, x1, y0, y1;            // its pixels, inside the framebuffer (inclusive)
     uint32_t on;
     uint32_t first;                    // number of its first tile row
-    uint32_t tileBase, tilesX, key;
-    uint32_t pad[7];
+    uint32_t tileBase, tilesX;
+    uint32_t key;
+    uint32_t count;                    // its covered pixels: 0 not counted, 1 lattice_pixels, 2 row_pixels
+    uint32_t right;                    // lattice_pixels: those of column xMax
+    float z[3], wInvSum, bound;        // depth_plane
 };
-static_assert(sizeof(BinRec) == 112, "seven 16-byte words");
+static_assert(sizeof(BinRec) == 112 && offsetof(BinRec, x0) == 48 && offsetof(BinRec, on) == 64 && offsetof(BinRec, key) == 80,
+              "seven 16-byte words, written word by word");
 
 // A tile row of a sub-triangle: a run of tiles.
 struct __align__(16) BinRow {
@@ -709,6 +756,116 @@ __device__ __forceinline__ void row_columns(const BinRec &r, uint32_t ty, int32_
     }
 }
 
+// The covered pixels of tile row ty, columns [lo, hi] (none is covered
+// outside them): per pixel row and edge the exact last column the edge
+// function leaves non-negative -- floor division of its value at x = 0 by
+// |ex|, found once in single precision and corrected by its remainder, then
+// stepped row by row with quotient and remainder.  Only for records whose
+// edge functions stay inside 32 bits (on).  A quotient beyond 2^21, which a
+// single correction may leave off, stays far outside the columns whatever
+// the rows add to it.
+__device__ __forceinline__ uint32_t row_pixels(const BinRec &r, uint32_t ty, int32_t lo, int32_t hi)
+{
+    const int32_t y0 = max(r.y0, (int32_t)(ty * PF_TILE)), y1 = min(r.y1, (int32_t)(ty * PF_TILE + PF_TILE - 1));
+    auto divide = [](int32_t v, int32_t d, float inv, int32_t &rem) {
+        int32_t q = __float2int_rd((float)v * inv);
+        rem = (int32_t)((uint32_t)v - (uint32_t)q * (uint32_t)d);
+        if (rem < 0) { q--; rem += d; }
+        if (rem >= d) { q++; rem -= d; }
+        return q;
+    };
+    int32_t q[3], rem[3], qs[3], rs[3], d[3];
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        d[e] = abs(r.ex[e]);
+        if (d[e] == 0) {
+            // a horizontal edge's rows are wholly inside or outside: the
+            // rows from the edge times 2^14, and 2^13 (columns stay below it)
+            const int32_t v = r.c[e] + r.ey[e] * y0;
+            q[e] = __float2int_rn((float)v * __frcp_rn(fabsf((float)r.ey[e]))) * (1 << 14) + (1 << 13);
+            qs[e] = r.ey[e] > 0 ? 1 << 14 : -(1 << 14);
+            rem[e] = rs[e] = 0; d[e] = 0x7fffffff;
+            continue;
+        }
+        const float inv = fabsf(r.rex[e]);
+        q[e] = divide(r.c[e] + r.ey[e] * y0, d[e], inv, rem[e]);
+        qs[e] = divide(r.ey[e], d[e], inv, rs[e]);
+    }
+    uint32_t n = 0;
+    for (int32_t y = y0; y <= y1; y++) {
+        int32_t a = lo, b = hi;
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            if (r.ex[e] > 0) a = max(a, -q[e]); else b = min(b, q[e]);
+            q[e] += qs[e]; rem[e] += rs[e];
+            if (rem[e] >= d[e]) { rem[e] -= d[e]; q[e]++; }
+        }
+        n += (uint32_t)max(b - a + 1, 0);
+    }
+    return n;
+}
+
+// The depth plane of a record.
+__device__ __forceinline__ float4 depth_plane(const BinRec &R)
+{
+    const float inf = __int_as_float(0x7f800000);
+    float4 p = make_float4(inf, 0.0f, 0.0f, R.bound);
+    if (!(fabsf(R.bound) < inf) || (R.x1 - R.x0 < PF_TILE && R.y1 - R.y0 < PF_TILE)) return p;
+    float m = 0.0f;
+    p.x = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        const float zw = R.z[e] * R.wInvSum, fc = (float)R.c[e], fx = (float)R.ex[e], fy = (float)R.ey[e];
+        p.x += fc * zw; p.y += fx * zw; p.z += fy * zw;
+        m += (fabsf(fc) + fabsf(fx) * (float)(R.x1 + PF_TILE) + fabsf(fy) * (float)(R.y1 + PF_TILE)) * fabsf(zw);
+    }
+    p.x += 4e-6f * m;
+    return p;
+}
+
+// The covered pixels of a record whose box is that of its vertices and whose
+// edge functions stay inside 32 bits: the vertices are pixels, and the
+// pixels where no edge function is negative are those of the closed
+// triangle -- by Pick's theorem half its doubled area and of its boundary's
+// pixels, and one -- less those of the column xMax, which the box leaves
+// out.  A boundary's pixels are the greatest common divisors of its edges'
+// components (Euclid's algorithm on the three at once; values below 2^14,
+// so a quotient in single precision is at most one off).
+__device__ __forceinline__ uint32_t lattice_pixels(const BinRec &R)
+{
+    int32_t a[3], b[3];
+#pragma unroll
+    for (int e = 0; e < 3; e++) { a[e] = abs(R.ex[e]); b[e] = abs(R.ey[e]); }
+    while ((b[0] | b[1] | b[2]) != 0) {
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            const int32_t q = (int32_t)__fdividef((float)a[e], (float)b[e]);
+            int32_t r = a[e] - q * b[e];
+            if (r < 0) r += b[e]; else if (r >= b[e]) r -= b[e];
+            if (b[e] != 0) { a[e] = b[e]; b[e] = r; }
+        }
+    }
+    return (uint32_t)((R.c[0] + R.c[1] + R.c[2] + a[0] + a[1] + a[2]) / 2 + 1) - R.right;
+}
+
+// The covered pixels of the warp's records whose box was cut (count 2; few
+// are), one after the other, a lane a tile row; returns the lane's share.
+__device__ __noinline__ uint32_t clipped_pixels(const BinWarp &S, uint32_t records)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t pixels = 0;
+    for (uint32_t k = 0; k < records; k++) {
+        const BinRec &r = S.rec[k];
+        if (r.count != 2u) continue;
+        for (uint32_t ty = (uint32_t)r.y0 / PF_TILE + lane; ty <= (uint32_t)r.y1 / PF_TILE; ty += 32u) {
+            int32_t lo, hi;
+            row_columns(r, ty, lo, hi);
+            if (lo <= hi) pixels += row_pixels(r, ty, lo, hi);
+        }
+    }
+    return pixels;
+}
+
 // Warp-cooperative binning of the lanes' sub-triangles: the tile rows of all
 // of them are numbered through and each lane takes one, finding the run of
 // tiles the sub-triangle may cover there; then the (row, tile) pairs of 32
@@ -729,7 +886,7 @@ __device__ __forceinline__ void row_columns(const BinRec &r, uint32_t ty, int32_
 // Every lane of the warp must call it (lanes with nothing to bin pass
 // has = false).
 #define BIN_BURST 4
-__device__ void bin_prim_warp(const BinArgs &B, const TileSpace &T, bool has, const PFPrim &P, uint32_t key, BinWarp &S)
+__device__ void bin_prim_warp(const BinArgs &B, const TileSpace &T, bool has, const PFPrim &P, bool on, uint32_t key, BinWarp &S)
 {
     const uint32_t all = 0xffffffffu;
     uint32_t tx0 = 0, ty0 = 0, ntx = 1, nty = 0;
@@ -739,15 +896,30 @@ __device__ void bin_prim_warp(const BinArgs &B, const TileSpace &T, bool has, co
     uint32_t rows;
     const uint32_t firstRow = warp_offsets(nty, rows);
     const uint32_t owners = __ballot_sync(all, nty > 0);
+    bool counts = false;
     if (nty > 0) {
-        const EdgeTest E = edge_test(P, T.W, T.H);
-        BinRec r;
-        for (int e = 0; e < 3; e++) { r.ex[e] = E.ex[e]; r.ey[e] = E.ey[e]; r.c[e] = E.c[e]; r.rex[e] = __frcp_rn((float)E.ex[e]); }
-        r.x0 = P.xMin; r.x1 = (int32_t)min((uint32_t)P.xMax, T.W) - 1;
-        r.y0 = P.yMin; r.y1 = (int32_t)min((uint32_t)P.yMax, T.H - 1u);
-        r.on = E.on; r.first = firstRow;
-        r.tileBase = T.tileBase; r.tilesX = T.tilesX; r.key = key;
-        S.rec[__popc(owners & lt)] = r;
+        // (16 bytes at a time as they are known: the record in registers
+        // beside P would spill)
+        int4 *q = reinterpret_cast<int4 *>(&S.rec[__popc(owners & lt)]);
+        q[3] = make_int4(P.xMin, (int32_t)min((uint32_t)P.xMax, T.W) - 1, P.yMin, (int32_t)min((uint32_t)P.yMax, T.H - 1u));
+        q[4] = make_int4(on, (int32_t)firstRow, (int32_t)T.tileBase, (int32_t)T.tilesX);
+        if (P.flags & (PFP_KIND | PFP_COUNT)) {
+            // no bound, nothing to count here
+            const float inf = __int_as_float(0x7f800000);
+            q[5] = make_int4((int32_t)key, 0, 0, 0);
+            B.planes[key >> PF_SUB_BITS] = make_float4(inf, 0.0f, 0.0f, raises_depth(P.rstate) ? __int_as_float(0x7fffffff) : inf);
+        } else {
+            const bool r1 = P.x1 == P.xMax, r2 = P.x2 == P.xMax, r3 = P.x3 == P.xMax;
+            const int32_t right = 1 + (r1 && r2 ? abs(P.y1 - P.y2) : r2 && r3 ? abs(P.y2 - P.y3) : r1 && r3 ? abs(P.y3 - P.y1) : 0);
+            counts = true;
+            q[5] = make_int4((int32_t)key, whole_box(P, T) ? 1 : 2, right, __float_as_int(P.z1));
+            q[6] = make_int4(__float_as_int(P.z2), __float_as_int(P.z3), __float_as_int(P.wInvSum), __float_as_int(depth_bound(P)));
+        }
+        const EdgeTest E = edge_test(P, on);
+        q[0] = make_int4(E.ex[0], E.ex[1], E.ex[2], E.ey[0]);
+        q[1] = make_int4(E.ey[1], E.ey[2], E.c[0], E.c[1]);
+        q[2] = make_int4(E.c[2], __float_as_int(__frcp_rn((float)E.ex[0])), __float_as_int(__frcp_rn((float)E.ex[1])),
+                         __float_as_int(__frcp_rn((float)E.ex[2])));
     }
     __syncwarp();
     for (uint32_t r0 = 0; r0 < rows; r0 += 32u) {
@@ -803,6 +975,21 @@ __device__ void bin_prim_warp(const BinArgs &B, const TileSpace &T, bool has, co
         }
         __syncwarp();                                          // the rows are free
     }
+    // the depth planes and the fragments, once the entries are on their way
+    // (read back from shared memory: held through the loops above they
+    // would spill)
+    if (!__any_sync(all, counts)) return;
+    const uint32_t records = __popc(__ballot_sync(all, nty > 0));
+    uint32_t count = 0, pixels = 0;
+    if (lane < records) {
+        const BinRec &r = S.rec[lane];
+        count = r.count;
+        if (count) B.planes[r.key >> PF_SUB_BITS] = depth_plane(r);
+        if (count == 1u) pixels = lattice_pixels(r);
+    }
+    if (__any_sync(all, count == 2u)) pixels += clipped_pixels(S, records);
+    pixels = __reduce_add_sync(all, pixels);
+    if (lane == 0 && pixels) atomicAdd(&B.cnt->batchFragments, (unsigned long long)pixels);
 }
 
 __device__ __forceinline__ void store_phong(PFPrimPhong *dst, const SVert &a, const SVert &b, const SVert &c)
@@ -980,6 +1167,7 @@ __device__ __noinline__ void clip_item(const PFDrawState &S, int stateIdx, const
     for (int i = 0; i < nsub; i++) {
         PFPrim P;
         if (!setup_prim(S, face, true, s[0], s[i + 1], s[i + 2], stateIdx, P)) continue;
+        P.flags |= PFP_COUNT;
         row_info_add(rows, (uint32_t)i, P);
         atomicAdd(&B.cnt->batchRasterized, 1ull);
         if (i == 0) { first = P; firstSet = true; }
@@ -994,6 +1182,10 @@ __device__ __noinline__ void clip_item(const PFDrawState &S, int stateIdx, const
     if (!firstSet) { first.flags = 0; first.xMin = 1; first.xMax = 0; }
     first.poolBase = (int32_t)base;
     O.prims[g] = first;
+    {
+        const float inf = __int_as_float(0x7f800000);      // (its pieces have no bound)
+        B.planes[g] = make_float4(inf, 0.0f, 0.0f, raises_depth(raster_state(S)) ? __int_as_float(0x7fffffff) : inf);
+    }
     if (O.rowInfo) O.rowInfo[g] = rows;
     if (firstSet && (S.flags & PFS_PHONG)) store_phong(&O.primsPh[g], s[0], s[1], s[2]);
 }
@@ -1007,7 +1199,7 @@ __device__ __noinline__ void clip_item(const PFDrawState &S, int stateIdx, const
 __device__ __forceinline__ bool item_setup(const PFSegment &sg, const PFDrawState *sState,
                                            const PFDrawState *__restrict__ states,
                                            const PFVertexOut *__restrict__ vout, uint32_t g, const ItemOut &O,
-                                           const BinArgs &B, const TileSpace &T, PFPrim &P)
+                                           const BinArgs &B, const TileSpace &T, PFPrim &P, bool &on)
 {
     const PFDrawState &S = sState ? *sState : states[sg.state];
     const uint32_t k = g - sg.itemBase + sg.itemSkip;
@@ -1068,6 +1260,14 @@ __device__ __forceinline__ bool item_setup(const PFSegment &sg, const PFDrawStat
     const bool kept = setup_prim(S, face, !is2D, s[0], s[1], s[2], sg.state, P);
     if (O.rowInfo) store_row_info(O.rowInfo, g, P, kept);
     if (!kept) return false;
+    // Who counts the record's covered pixels: k_raster, visiting them, where
+    // the edge functions may wrap, where k_rows draws, and for triangles
+    // within 32x32 pixels of launches with fewer than 8 items a tile, whose
+    // tiles seldom hold a second batch to drop records from (with a limit of
+    // 8x8 pixels sphere1080's k_items took 22.6 us, now 21.3; without
+    // counting 20.0); the others here.
+    on = edge_on(P, T.W, T.H);
+    if (T.rows || !on || (!B.countSmall && P.xMax - P.xMin <= 4 * PF_TILE && P.yMax - P.yMin < 4 * PF_TILE)) P.flags |= PFP_COUNT;
     O.prims[g] = P;
     if (S.flags & PFS_PHONG) store_phong(&O.primsPh[g], s[0], s[1], s[2]);
     return true;
@@ -1097,14 +1297,14 @@ __global__ void __launch_bounds__(128, 6) k_items(const PFSegment *__restrict__ 
     const int su = sUniform;
     // every lane stays to the end: binning below is warp-cooperative
     PFPrim P;
-    bool kept = false;
-    TileSpace T{ 0, 0, 0, 0 };
+    bool kept = false, on = false;
+    TileSpace T{ 0, 0, 0, 0, false };
     if (g < nItems) {
         // the segment and its draw state are read in place (one address for
         // the block: L1 serves it after the first access)
         const PFSegment &sg = segs[su >= 0 ? su : seg_of_item(segs, nSegs, g)];
         T = tile_space(B, sg.target);
-        kept = item_setup(sg, nullptr, states, vout, g, O, B, T, P);
+        kept = item_setup(sg, nullptr, states, vout, g, O, B, T, P, on);
     }
     // one counter update per warp, its result unused (a reduction in L2, no
     // round trip, no block barrier)
@@ -1114,7 +1314,7 @@ __global__ void __launch_bounds__(128, 6) k_items(const PFSegment *__restrict__ 
         const uint64_t grp = row_group(g < nItems ? O.rowInfo[g] : 0ull);
         if ((threadIdx.x & 31) == 0) O.rowGroup[g >> 5] = grp;
     }
-    bin_prim_warp(B, T, kept, P, g << PF_SUB_BITS, sBin[warp]);
+    bin_prim_warp(B, T, kept, P, on, g << PF_SUB_BITS, sBin[warp]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1131,14 +1331,13 @@ __global__ void __launch_bounds__(128, 6) k_items(const PFSegment *__restrict__ 
 // submission order:
 //   1. every lane loads one record of the batch into the warp's shared
 //      memory and derives its edge functions at the tile origin and its
-//      bounding box clipped to the tile;
-//   2. from the second batch on, records that lie behind every pixel of the
-//      tile are dropped (their covered pixels still count); each lane walks
-//      the others in order at its own two pixels: coverage with the
-//      reference's integer edge functions, depth, depth test and depth write
-//      (triangles.c:398-438) -- which leaves, per pixel, the fragments that
-//      passed and are not replaced by a later unblended one (bit k of a
-//      32-bit mask: the record's place in the batch);
+//      bounding box clipped to the tile (from the second batch on, records
+//      that lie behind every pixel of the tile do not get into a batch);
+//   2. each lane walks the records in order at its own two pixels: coverage
+//      with the reference's integer edge functions, depth, depth test and
+//      depth write (triangles.c:398-438) -- which leaves, per pixel, the
+//      fragments that passed and are not replaced by a later unblended one
+//      (bit k of a 32-bit mask: the record's place in the batch);
 //   3. the passing fragments are listed pixel by pixel in submission order
 //      and shaded densely over the warp (texture, Gouraud / Phong colour:
 //      the source colour does not depend on the destination);
@@ -1168,6 +1367,7 @@ struct RasterArgs {
     uint32_t cap;
     const PFPrim *prims;
     const PFPrimPhong *primsPh;
+    const float4 *planes;
     const PFPrim *pool;
     const PFPrimPhong *poolPh;
     const PFDrawState *states;
@@ -1202,14 +1402,18 @@ struct __align__(16) QEdge {
     float zReject;             // every covered fragment fails the depth test when zReject >= depth (NaN: never)
 };
 
+#define QE_COUNT (1u << 18)     // of box: k_raster counts the record's fragments (k_items has not; rectangles have none)
+
 // Shared memory of one warp.
 struct QWarp {
     SPrim rec[QCHN];
     QEdge edge[QCHN];
-    uint32_t keys[REG_SORT_MAX];   // a short bin's keys in submission order (sorted in registers)
+    uint32_t keys[REG_SORT_MAX];   // the queue of the next keys; a short bin's further ones, sorted in registers
     uint32_t pend[PF_TILE_PIXELS]; // per pixel (32 slot + lane) the bin key of its fragment that waits to be shaded
     uint16_t fdesc[QFW];       // listed fragments: tile pixel << 5 | record
     uint32_t fc[QFW];          // their colour
+    uint32_t queued, lowering; // queue_refill: keys in the queue; no key so far may raise a depth
+    uint32_t pad[2];
 };
 
 // Edge set-up of a record (its first three 16-byte words: x1 y1 x2 y2 |
@@ -1241,7 +1445,8 @@ __device__ __forceinline__ void tile_edge(const int4 q0, const int4 q1, const in
     E.e0[0] = e0[0]; E.e0[1] = e0[1]; E.e0[2] = e0[2];
     E.ex0 = sx[0]; E.ex1 = sx[1]; E.ex2 = sx[2];
     E.ey0 = sy[0]; E.ey1 = sy[1]; E.ey2 = sy[2];
-    E.box = bx0 | (bw << 4) | (by0 << 8) | (bh << 12) | (((flags & PFP_KIND) >> 6) << 16);
+    E.box = bx0 | (bw << 4) | (by0 << 8) | (bh << 12) | (((flags & PFP_KIND) >> 6) << 16) |
+            (((flags & PFP_KIND) ? (flags & PFP_KIND) != PFP_BLIT : (flags & PFP_COUNT) != 0) ? QE_COUNT : 0u);
     E.rstate = rstate;
     E.zReject = zReject;
 }
@@ -1252,54 +1457,6 @@ __device__ __forceinline__ uint32_t depth_key(float d)
 {
     const uint32_t u = (uint32_t)__float_as_int(d);
     return d != d ? 0xffffffffu : u ^ ((int32_t)u < 0 ? 0xffffffffu : 0x80000000u);
-}
-
-// A tile's depth-test rejection bound of a record whose box reaches past
-// the tile (depth_reject_bound, over the tile's part of the box instead of
-// the whole triangle).  The interpolated term zs is affine in the pixel, so
-// over the box it is at most its value at one corner plus the steps to the
-// largest one; m bounds the sum of the absolute terms, and 2e-6 m the
-// rounding of this evaluation (a dozen operations of 2^-24 each) and of a
-// covered fragment's own terms (their sum there is at most m).  The
-// corners' depths of a wide triangle say little about its depth in one tile:
-// with this bound most records behind the tile's pixels are dropped whole
-// (k_raster: 64-soup batch 3,017 -> 1,925 us, soup256 139 -> 65 us).  zq:
-// wInvSum, z1, z2, z3.
-__device__ __forceinline__ float tile_reject(const QEdge &E, const float4 zq)
-{
-    const float bound = E.zReject;
-    if (!(bound == bound)) return bound;                     // no bound: func, depth test or signs
-    const uint32_t bx0 = E.box & 15u, bw = (E.box >> 4) & 15u, by0 = (E.box >> 8) & 15u, bh = (E.box >> 12) & 15u;
-    const float dx = (float)bw - 1.0f, dy = (float)bh - 1.0f;
-    const int32_t ex[3] = { E.ex0, E.ex1, E.ex2 }, ey[3] = { E.ey0, E.ey1, E.ey2 };
-    const float z[3] = { zq.y, zq.z, zq.w };
-    float a = 0.0f, gx = 0.0f, gy = 0.0f, m = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 3; e++) {
-        const int32_t w = (int32_t)((uint32_t)E.e0[e] + bx0 * (uint32_t)ex[e] + by0 * (uint32_t)ey[e]);
-        const float zw = z[e] * zq.x, fw = (float)w, fx = (float)ex[e], fy = (float)ey[e];
-        a += fw * zw; gx += fx * zw; gy += fy * zw;
-        m += (fabsf(fw) + fabsf(fx) * dx + fabsf(fy) * dy) * fabsf(zw);
-    }
-    const float top = a + fmaxf(gx * dx, 0.0f) + fmaxf(gy * dy, 0.0f) + 2e-6f * m;
-    const float lo = fminf(z[0], fminf(z[1], z[2])), hi = fminf(top, fmaxf(z[0], fmaxf(z[1], z[2])));
-    float b;
-    if (lo > 0.0f) {
-        if (!(hi > 0.0f)) return bound;
-        b = __frcp_rn(hi * 1.00001f) * 0.9999899f;
-    } else {
-        if (!(hi < 0.0f)) return bound;
-        b = __frcp_rn(hi * 0.99999f) * 1.0000101f;
-    }
-    return fabsf(b) < 1e30f ? fmaxf(b, bound) : bound;
-}
-
-// Whether the record may raise a pixel's depth (a batch without such
-// records only lowers depths).
-__device__ __forceinline__ bool raises_depth(uint32_t rstate)
-{
-    const uint32_t func = (rstate >> 16) & 255u;
-    return (rstate & PFS_DEPTH_MASK) && !((rstate & PFS_DEPTH_TEST) && (func == 2u || func == 3u || func == 0u));
 }
 
 // Normalised weights and depth of a covered fragment at tile pixel (X, Y)
@@ -1682,6 +1839,55 @@ __device__ __forceinline__ void tile_list(unsigned long long m, uint32_t off, ui
     }
 }
 
+// Refill the queue of a tile's next keys at Q.keys (`left` of them at
+// Q.keys[taken] on) from the bin's keys c0 .. n - 1 (at Q.keys too when bin
+// is null) up to a batch, leaving out the records that lie behind every
+// pixel of the tile -- its farthest depth is farKey -- by their depth planes
+// alone: 16 bytes and a dozen operations a key, where copying the record,
+// its set-up and its coverage take 30.  Their covered pixels need no visit,
+// k_items has counted them.  Nothing is left out once a key came that may
+// raise a depth.  Returns the next key.  Against dropping them after their
+// set-up: 64-soup batch 1,458 -> 1,160 us, phong1080 315 -> 256, the
+// 2,000-triangle soup at 256x256 50 -> 47, sphere1080, whose tiles hold one
+// batch, unchanged; k_items pays for the counting (batch 326 -> 331,
+// phong1080 190 -> 230, sphere1080 20 -> 21.3).  Two groups of 32 keys a
+// step: 1,209 -> 1,259; out of line: 1,190.
+__device__ __forceinline__ uint32_t queue_refill(QWarp &Q, const uint32_t *bin, const float4 *planes, uint32_t n, uint32_t c0,
+                                              uint32_t left, uint32_t taken, uint32_t farKey, uint32_t ox, uint32_t oy)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t k = lane < left ? Q.keys[taken + lane] : 0u;
+    __syncwarp();
+    if (lane < left) Q.keys[lane] = k;
+    uint32_t queued = left;
+    bool lowering = Q.lowering != 0;
+    const float farDepth = __int_as_float((int32_t)((farKey & 0x80000000u) ? farKey ^ 0x80000000u : ~farKey));
+    // (no bound below 3e38: a record without one has none either)
+    const float inv = farDepth > 0.0f ? fminf(__frcp_rn(farDepth) * 0.99999f, 3e38f) :
+                      farDepth < 0.0f ? __frcp_rn(farDepth) * 1.00001f : __int_as_float(0x7fffffff);
+    const float fx = (float)ox, fy = (float)oy;
+    while (queued < QCHN && c0 < n) {
+        const uint32_t i = c0 + lane;
+        uint32_t key = 0;
+        float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < n) {
+            key = bin ? __ldg(bin + i) : Q.keys[i];
+            p = __ldg(planes + (key >> PF_SUB_BITS));
+        }
+        lowering = __all_sync(0xffffffffu, p.w == p.w) && lowering;
+        const float top = fminf(((p.x + p.y * fx) + p.z * fy) + (fmaxf(p.y * 7.0f, 0.0f) + fmaxf(p.z * 7.0f, 0.0f)), p.w);
+        const bool behind = lowering && top <= inv && (p.w > 0.0f) == (inv > 0.0f) && (key & ((1u << PF_SUB_BITS) - 1u)) == 0;
+        const uint32_t m = __ballot_sync(0xffffffffu, i < n && !behind);
+        if ((m >> lane) & 1u) Q.keys[queued + __popc(m & ((1u << lane) - 1u))] = key;
+        queued += __popc(m);
+        c0 += 32u;
+        __syncwarp();
+    }
+    if (lane == 0) { Q.queued = queued; Q.lowering = lowering; }
+    __syncwarp();
+    return c0;
+}
+
 // GEN: a target is not RGBA / unsigned byte.  PHONG: a draw state lights per
 // fragment; without that code nothing spills: sphere1080 58 -> 56 us,
 // 64-soup batch 1,925 -> 1,780.  Warps an SM, by what fits without spills:
@@ -1699,7 +1905,10 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
     asm volatile("griddepcontrol.wait;" ::: "memory");   // k_binsort is done
     if (a.cnt->abortCommand <= a.command) return;
     // the batch completed set-up without overflow: its sub-triangles count
-    if (blockIdx.x == 0 && tid == 0) atomicAdd(&a.cnt->rasterized, a.cnt->batchRasterized);
+    if (blockIdx.x == 0 && tid == 0) {
+        atomicAdd(&a.cnt->rasterized, a.cnt->batchRasterized);
+        atomicAdd(&a.cnt->fragments, a.cnt->batchFragments);
+    }
     const uint32_t lx = (uint32_t)lane & 7u, ly = (uint32_t)lane >> 3;     // my pixels: (lx, ly) and (lx, ly + 4)
     uint32_t frags = 0;                                // (at most 64 a bin entry and tile)
 
@@ -1892,24 +2101,33 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
     // lanes' own; it ends the waiting, so that draws that alternate between
     // blended and unblended records pay for it once a tile.
     bool defer = n > QCHN, pending = false;
-    uint32_t ph = 0, c0 = 0;
+    uint32_t ph = 0;
+    // The bin's next keys, in order, are a queue at Q.keys: a batch is its
+    // first 32 (queue_refill).  A short bin's keys wait behind the queue:
+    // c0, the next one, is never below its room.
+    uint32_t c0 = min(n, (uint32_t)QCHN), queued = c0, taken = 0;
+    if (lane == 0) Q.lowering = 1;
+    if (!regSort) Q.keys[lane] = __ldg(bin + lane);
+    __syncwarp();
     for (;;) {
-        if (ph == 0 && c0 >= n) {
+        if ((!PHONG || ph == 0) && taken) {
+            if ((!PHONG || !pending) && queued == taken && c0 >= n) break;
+            const uint32_t farKey = __reduce_max_sync(0xffffffffu, max(in0 ? depth_key(dep0) : 0u, in1 ? depth_key(dep1) : 0u));
+            c0 = queue_refill(Q, regSort ? nullptr : bin, a.planes, n, c0, queued - taken, taken, farKey, ox, oy);
+            queued = Q.queued; taken = 0;
+        }
+        if (ph == 0 && queued == 0) {
             if (!PHONG || !pending) break;
             ph = 1;
         }
         const uint32_t phase = PHONG ? ph : 0u;
-        // the farthest depth of the tile's pixels, from the second batch on
-        // (a tile of one batch has nothing in front yet)
-        const uint32_t farKey = c0 == 0 || phase != 0 ? 0xffffffffu :
-            __reduce_max_sync(0xffffffffu, max(in0 ? depth_key(dep0) : 0u, in1 ? depth_key(dep1) : 0u));
         // 1. my record: load, stage, derive its tile set-up and coverage
         uint32_t kind = 0;
         uint32_t covLo = 0, covHi = 0;                  // its coverage, rows 0-3 and 4-7 (bit 8 y + x of the 64)
-        bool raises = false, hidden = false, blends = false;
+        bool blends = false;
         uint32_t key = 0xffffffffu;
         if (phase != 0) key = Q.pend[32u * (phase - 1u) + (uint32_t)lane];
-        else if (c0 + (uint32_t)lane < n) key = regSort ? Q.keys[c0 + (uint32_t)lane] : __ldg(bin + c0 + lane);
+        else if ((uint32_t)lane < queued) key = Q.keys[lane];
         const bool have = key != 0xffffffffu;
         if (have) {
             const uint32_t item = key >> PF_SUB_BITS, sub = key & ((1u << PF_SUB_BITS) - 1);
@@ -1929,7 +2147,6 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
             QEdge E;
             tile_edge(r[0], r1, r2, Q.rec[lane].p.rstate, Q.rec[lane].p.zReject, ox, oy, W, H, E);
             kind = (uint32_t)r2.z & PFP_KIND;
-            raises = raises_depth(E.rstate);
             blends = (E.rstate & PFS_BLEND) != 0;
             // my record's coverage of the tile: the pixels of its box that
             // pass the integer edge test (triangles.c:398-424) or, for a
@@ -1976,9 +2193,6 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                         r0 += (uint32_t)E.ey0; r1 += (uint32_t)E.ey1; r2 += (uint32_t)E.ey2;
                     }
                 }
-                if (n > QCHN && ((uint32_t)r2.x - (uint32_t)r1.z > bw || (uint32_t)r2.y - (uint32_t)r1.w >= bh))
-                    E.zReject = tile_reject(E, reinterpret_cast<const float4 *>(r)[3]);
-                hidden = E.zReject == E.zReject && depth_key(E.zReject) >= farKey;
             } else {
                 const PFPrim &P = Q.rec[lane].p;
                 for (uint32_t y = by0; y < by0 + bh; y++)
@@ -1995,18 +2209,9 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
             if (phase == 1) vis0 = have ? 1u << lane : 0u; else vis1 = have ? 1u << lane : 0u;
             __syncwarp();
         } else {
-        // a record behind every pixel of the tile has no fragment that passes
-        // (no record of the batch raises a depth): its covered pixels count,
-        // and that is all
-        const bool lowers = __all_sync(0xffffffffu, !raises);
-        const bool live = (covLo | covHi) != 0 && !(lowers && hidden);
+        const bool live = (covLo | covHi) != 0;
         if (PHONG && pending && __any_sync(0xffffffffu, live && blends)) { ph = 1; __syncwarp(); continue; }
-        if (!live) {
-            // (a half tile: its own rows)
-            frags += (whole || rowA == ly ? __popc(covLo) : 0) + (whole || rowA != ly ? __popc(covHi) : 0);
-            covLo = covHi = 0;
-        }
-        if (!__any_sync(0xffffffffu, live)) { c0 += QCHN; continue; }
+        if (!__any_sync(0xffffffffu, live)) { taken = min(queued, (uint32_t)QCHN); __syncwarp(); continue; }
         __syncwarp();
         // 2a. coverage per pixel: bit k of cm0 / cm1 -- record k covers my
         //     pixel of slot 0 / 1 -- the records' masks transposed over the
@@ -2027,8 +2232,8 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                 const uint32_t box = (uint32_t)q2.y, rs = (uint32_t)q2.z;
                 const int func = (int)((rs >> 16) & 255u);
                 float z;
+                cov += (box >> 18) & 1u;
                 if (((box >> 16) & 3u) == 0) {
-                    cov++;
                     if (__int_as_float(q2.w) >= d) continue;  // every fragment of it fails the depth test
                     const int4 q0 = e4[0], q1 = e4[1];
                     const uint32_t w1 = (uint32_t)q0.x + lx * (uint32_t)q0.w + row * (uint32_t)q1.z;
@@ -2045,7 +2250,6 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                     // a point, line or rectangle set up on the host: its own
                     // depth, the scalar depth test (rectangles are not fragments)
                     const PFPrim &P = Q.rec[k].p;
-                    if (((box >> 16) & 3u) != (PFP_BLIT >> 6)) cov++;
                     z = lp_depth(P, (int32_t)X0, (int32_t)Y);
                     if ((rs & PFS_DEPTH_TEST) && !depth_sisd(func, z, d)) continue;
                 }
@@ -2065,8 +2269,7 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
             const bool d0 = waits(vis0), d1 = waits(vis1);
             if (__any_sync(0xffffffffu, d0 || d1)) {
                 auto key_of = [&](uint32_t vis) {
-                    const uint32_t i = c0 + (uint32_t)(__ffs(vis) - 1);
-                    return regSort ? Q.keys[i] : __ldg(bin + i);
+                    return Q.keys[__ffs(vis) - 1];
                 };
                 if (d0 || !pending) Q.pend[lane] = d0 ? key_of(vis0) : 0xffffffffu;
                 if (d1 || !pending) Q.pend[32 + lane] = d1 ? key_of(vis1) : 0xffffffffu;
@@ -2119,7 +2322,7 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
             __syncwarp();                                  // the window's lists are free
         }
         __syncwarp();                                      // the batch's records are free
-        if (phase == 0) c0 += QCHN;
+        if (phase == 0) taken = min(queued, (uint32_t)QCHN);
         else if (phase == 1 && whole) ph = 2;
         else { ph = 0; pending = false; defer = false; }
     }
@@ -2762,7 +2965,8 @@ cudaError_t pfd_launch_vertex(const PFBatchLaunch &L, cudaStream_t st)
 cudaError_t pfd_launch_items(const PFBatchLaunch &L, cudaStream_t st)
 {
     if (L.nItems == 0) return cudaSuccess;
-    BinArgs B{ L.binCount, L.tileList, L.listStride, L.bins, L.cap, L.targets, L.cnt, L.command };
+    BinArgs B{ L.binCount, L.tileList, L.listStride, L.bins, L.cap, L.targets, L.cnt, L.command, L.planes,
+               L.nItems / 8u >= L.totalTiles };
     ItemOut O{ L.prims, L.primsPh, L.pool, L.poolPh, L.poolCap, L.rowCount ? L.rowInfo : nullptr, L.rowGroup };
     // Items a warp: a full warp of 32 sets up fastest, but a small launch
     // then leaves most of the GPU idle while a few warps bin all its tiles.
@@ -2788,7 +2992,7 @@ static size_t raster_smem(int warps)
 
 static RasterArgs raster_args(const PFBatchLaunch &L)
 {
-    return RasterArgs{ L.binCount, L.tileList, L.listStride, L.bins, L.cap, L.prims, L.primsPh, L.pool, L.poolPh, L.states,
+    return RasterArgs{ L.binCount, L.tileList, L.listStride, L.bins, L.cap, L.prims, L.primsPh, L.planes, L.pool, L.poolPh, L.states,
                        L.targets, L.nTargets, L.totalTiles, L.cnt, L.command, L.anyPhong, 0 };
 }
 

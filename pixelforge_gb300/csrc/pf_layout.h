@@ -148,6 +148,7 @@ typedef struct PF_ALIGN16 {
  * which stand in for the draw state's (same bit positions as PFS_*). */
 enum {
     PFP_Y_LONGER = 1u << 2,       /* lines: y is the long axis */
+    PFP_COUNT = 1u << 2,          /* triangles: k_raster counts the fragments (else k_items has) */
     PFP_BLEND = 1u << 3,          /* blend (scalar rules) */
     PFP_DEPTH_TEST = 1u << 4,     /* depth-test (scalar rules) */
     PFP_DEPTH_WRITE = 1u << 5,    /* write depth */
@@ -209,6 +210,7 @@ typedef struct {
     unsigned int maxBin;          /* largest tile bin count seen */
     unsigned int clipCount;       /* clipped sub-triangles allocated */
     unsigned long long batchRasterized;   /* sub-triangles set up by the current batch */
+    unsigned long long batchFragments;    /* and their covered pixels, of those k_items counts */
     unsigned int tileQueue;       /* next entry of the current batch's raster work list */
     unsigned int sortQueue;       /* next entry of the current batch's bin-sort list */
     unsigned int tileListCount;   /* tiles with a non-empty bin, listed by the binning */

@@ -45,7 +45,8 @@ constexpr size_t kOffCnt = align256(kOffSeg + sizeof(PFSegment));
 constexpr size_t kOffTarget = align256(kOffCnt + sizeof(PFDevCounters));
 constexpr size_t kOffVout = align256(kOffTarget + sizeof(PFTarget));
 constexpr size_t kOffPrims = align256(kOffVout + sizeof(PFVertexOut) * 3 * (size_t)kMaxTris);
-constexpr size_t kOffPool = align256(kOffPrims + sizeof(PFPrim) * (size_t)kMaxItems);
+constexpr size_t kOffPlanes = align256(kOffPrims + sizeof(PFPrim) * (size_t)kMaxItems);
+constexpr size_t kOffPool = align256(kOffPlanes + sizeof(float4) * (size_t)kMaxItems);
 constexpr size_t kOffPh = align256(kOffPool + sizeof(PFPrim) * (size_t)kPoolCap);
 // bin counters, then the raster's work lists (the non-empty tiles and those
 // of each heavy level), listStride entries each
@@ -152,6 +153,7 @@ extern "C" int pfgbDrawTrianglesStatic(const float *positions, const uint32_t *c
     L.states = (const PFDrawState *)(s + kOffState);
     L.vout = (PFVertexOut *)(s + kOffVout); L.nVerts = G.nVerts; L.nItems = L.itemSpan = G.nItems;
     L.prims = (PFPrim *)(s + kOffPrims); L.primsPh = (PFPrimPhong *)(s + kOffPh);
+    L.planes = (float4 *)(s + kOffPlanes);
     L.pool = (PFPrim *)(s + kOffPool); L.poolPh = (PFPrimPhong *)(s + kOffPh); L.poolCap = kPoolCap;
     L.binCount = (uint32_t *)(s + kOffBinCount); L.bins = (uint32_t *)(s + kOffBins); L.cap = kBinCap;
     L.listStride = kListStride; L.tileList = L.binCount + kListStride;
