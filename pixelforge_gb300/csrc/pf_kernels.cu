@@ -877,7 +877,9 @@ __device__ __noinline__ uint32_t clipped_pixels(const BinWarp &S, uint32_t recor
 // items covering hundreds of tiles each, 4.5 tiles tested per entry) took
 // 614 us, now 305; phong1080, whose triangles cover one or two tiles, 285
 // -> 217 us; the 2,000-triangle soup at 256x256 136 -> 17 us together with
-// the items a warp (pfd_launch_items).  Pairs of one window of
+// the items a warp (pfd_launch_items).  Planes and fragment counts added
+// since cost 5 us of the batch and 40 of phong1080, and save k_raster 300
+// and 59 (queue_refill).  Pairs of one window of
 // 32 that touch the same tile share one atomic on its counter (neighbouring
 // triangles of a mesh usually do), slots within a group follow lane order;
 // the pairs of a single sub-triangle are distinct tiles and skip the
