@@ -1864,8 +1864,12 @@ __device__ __forceinline__ uint32_t queue_refill(QWarp &Q, const uint32_t *bin, 
     uint32_t queued = left;
     bool lowering = Q.lowering != 0;
     const float farDepth = __int_as_float((int32_t)((farKey & 0x80000000u) ? farKey ^ 0x80000000u : ~farKey));
-    // (no bound below 3e38: a record without one has none either)
-    const float inv = farDepth > 0.0f ? fminf(__frcp_rn(farDepth) * 0.99999f, 3e38f) :
+    // No bound below 3e38: a record without one has none either.  NaN, which
+    // hides nothing, where the reciprocal of the farthest depth does not tell
+    // on which side of zero that is: for zeros and for infinities, before
+    // which every depth lies, negative ones too.
+    const float inv = !(fabsf(farDepth) < __int_as_float(0x7f800000)) ? __int_as_float(0x7fffffff) :
+                      farDepth > 0.0f ? fminf(__frcp_rn(farDepth) * 0.99999f, 3e38f) :
                       farDepth < 0.0f ? __frcp_rn(farDepth) * 1.00001f : __int_as_float(0x7fffffff);
     const float fx = (float)ox, fy = (float)oy;
     while (queued < QCHN && c0 < n) {
