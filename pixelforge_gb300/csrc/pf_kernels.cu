@@ -2162,13 +2162,16 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                 // (covered and visible already)
             } else if (kind == 0) {
                 // the whole box when no edge function is negative at its
-                // least corner (with these bounds none wraps inside the tile)
+                // least corner (values in [-2^30, 2^30) and steps in
+                // [-2^24, 2^24): none wraps inside the tile; compared as
+                // unsigned, since -2^31 has no absolute value)
                 bool full = bw + bh >= 12u;
                 if (full)
 #pragma unroll
                 for (int e = 0; e < 3; e++) {
                     const int32_t ex = e == 0 ? E.ex0 : e == 1 ? E.ex1 : E.ex2, ey = e == 0 ? E.ey0 : e == 1 ? E.ey1 : E.ey2;
-                    full = full && abs(E.e0[e]) < (1 << 30) && abs(ex) < (1 << 24) && abs(ey) < (1 << 24) &&
+                    full = full && (uint32_t)E.e0[e] + (1u << 30) < (1u << 31) && (uint32_t)ex + (1u << 24) < (1u << 25) &&
+                           (uint32_t)ey + (1u << 24) < (1u << 25) &&
                            E.e0[e] + (int32_t)(ex > 0 ? bx0 : bx0 + bw - 1u) * ex + (int32_t)(ey > 0 ? by0 : by0 + bh - 1u) * ey >= 0;
                 }
                 const uint32_t cols = ((1u << bw) - 1u) << bx0;
