@@ -1687,11 +1687,17 @@ bool flush(Renderer *r)
     // leading fused pfClear keeps travel here too: each was a copy of its own,
     // a launch and a switch between copy engine and kernels
     const int64_t countersOff = r->staging.alloc(sizeof(PFDevCounters));
+    // (not for copies of one PFframebuffer, which share its pixels: what was
+    // drawn through the other one before the clear is kept)
+    std::vector<const FBMirror *> sorted(mirrors.begin(), mirrors.end());
+    std::sort(sorted.begin(), sorted.end(), std::less<const FBMirror *>());
+    const bool copies = std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end();
     std::vector<int64_t> headOff(used.size(), -1);                 // 8 raw pixels, then 8 depths
     for (auto &o : ops)
         for (size_t k = 0; o.kind == 0 && k < o.targets.size(); k++) {
             const size_t u = slot.at(o.targets[k]);
-            if (o.clearCmd[k] >= 0 && o.clearCmd[k] == firstCmd[u] && cmds[o.clearCmd[k]].kind == CMD_CLEAR)
+            if (o.clearCmd[k] >= 0 && o.clearCmd[k] == firstCmd[u] && cmds[o.clearCmd[k]].kind == CMD_CLEAR &&
+                (!copies || std::count(mirrors.begin(), mirrors.end(), mirrors[u]) == 1))
                 headOff[u] = r->staging.alloc(8 * mirrors[u]->bpp + 8 * sizeof(float));
         }
     for (auto &rec : r->segs) {
