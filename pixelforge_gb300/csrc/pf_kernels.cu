@@ -30,9 +30,9 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <mutex>
 #include "pf_layout.h"
 #include "pf_device.h"
+#include "pf_limits.h"
 #include "pf_pixfmt.h"
 
 namespace {
@@ -3005,40 +3005,12 @@ static RasterArgs raster_args(const PFBatchLaunch &L)
                        L.targets, L.nTargets, L.totalTiles, L.cnt, L.command, L.anyPhong, 0 };
 }
 
-// CTAs of `kernel` that fit on an SM, its shared-memory limits set.  Asked of
-// the driver once per device, kernel and size: the three calls for every
-// launch of a frame take about as long as a small frame's kernel.
-static cudaError_t ctas_per_sm(const void *kernel, int block, size_t smem, bool maxShared, int &fit)
-{
-    struct Known { const void *kernel; int dev, block, fit; size_t smem; };
-    static std::mutex m;
-    static Known known[64];
-    static int count = 0;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(m);
-    size_t limit = 0;                                  // what the kernel's limit was raised to
-    for (int i = 0; i < count; i++) {
-        const Known &k = known[i];
-        if (k.kernel != kernel || k.dev != dev) continue;
-        if (k.block == block && k.smem == smem) { fit = k.fit; return cudaSuccess; }
-        limit = k.smem > limit ? k.smem : limit;
-    }
-    if (smem > limit) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && maxShared)                 // the CTAs' shared memory, not L1, bounds how many fit on an SM
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, block, smem);
-    if (e == cudaSuccess && count < 64) known[count++] = Known{ kernel, dev, block, fit, smem };
-    return e;
-}
-
 // Persistent grid of `kernel`: as many CTAs as fit on the GPU at once, at
 // most `perSM` per SM (0: as many as fit), at most `units`.
 static cudaError_t persistent_grid(const void *kernel, int block, size_t smem, bool maxShared, int perSM, uint32_t units, uint32_t &grid)
 {
     int fit = 0;
-    cudaError_t e = ctas_per_sm(kernel, block, smem, maxShared, fit);
+    cudaError_t e = pfd_ctas_per_sm(kernel, block, smem, maxShared, fit);
     if (e != cudaSuccess) return e;
     uint32_t per = (uint32_t)(fit > 0 ? fit : 1);
     if (perSM > 0) per = min(per, (uint32_t)perSM);
@@ -3085,12 +3057,12 @@ cudaError_t pfd_launch_raster(const PFBatchLaunch &L, cudaStream_t st)
     e = launch_serialized(kernel, grid, (unsigned)(warps * 32), smem, st, raster_args(L));
     if (e != cudaSuccess || L.rowCount == 0 || !L.rowInfo || !L.rowGroup) return e;
     const bool inSmem = L.rowMaxW <= ROW_SMEM_MAX_W;
-    const uint32_t rowW = (L.rowMaxW + 255u) & ~255u;                                   // (few sizes: ctas_per_sm keeps them)
+    const uint32_t rowW = (L.rowMaxW + 255u) & ~255u;                                   // (few sizes: pfd_ctas_per_sm keeps them)
     const size_t rsm = sizeof(RowShared) + (inSmem ? (size_t)rowW * 8 : 0);            // colour and depth of the row
     auto rows = inSmem ? (L.anyPhong ? k_rows<true, true> : k_rows<true, false>)
                        : (L.anyPhong ? k_rows<false, true> : k_rows<false, false>);
     int fit = 0;
-    e = ctas_per_sm((const void *)rows, ROW_THREADS, rsm, false, fit);
+    e = pfd_ctas_per_sm((const void *)rows, ROW_THREADS, rsm, false, fit);
     if (e != cudaSuccess) return e;
     return launch_serialized(rows, L.rowCount, ROW_THREADS, rsm, st, raster_args(L), L.segs, L.nSegs,
                              (const uint64_t *)L.rowInfo, (const uint64_t *)L.rowGroup, rowW);
