@@ -1981,7 +1981,7 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
     if (gt == 0xfffffffeu) continue;
     if (gt & 0x80000000u) {
         // the fused clear of the empty tiles of group gt: one tile a lane,
-        // each row of RGBA8 pixels and depths as two 16-byte stores
+        // each row of pixels and depths in 16-byte stores
         const uint32_t t = 32u * (gt & 0x7fffffffu) + (uint32_t)lane;
         if (t < a.totalTiles && __ldg(a.binCount + t) == 0) {
             int clo = 0, chi = a.nTargets - 1;
@@ -1991,15 +1991,26 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                 const uint32_t tile = t - C.tileBase;
                 const uint32_t cx = (tile % C.tilesX) * PF_TILE, cy = (tile / C.tilesX) * PF_TILE;
                 const uint32_t xe = min(cx + PF_TILE, C.W);
+                // (GEN: pixels of 2, 4, 8 or 16 bytes, the others pixel by pixel.
+                // Bound by the sectors L2 takes: a word a store, the sphere
+                // frame's raster sent it 14 M of RGBA float, most of them in part,
+                // and took 200 us with L2 full of written lines, 104 now; RGBA
+                // half 119 -> 105, 5-6-5 79 -> 71)
+                const uint32_t bytes = GEN ? (uint32_t)pff_bytes(C.fmt) : 4u;
+                const bool wide = !GEN || (bytes & (bytes - 1u)) == 0;
+                uint4 v = make_uint4(C.clearRaw[0], C.clearRaw[0], C.clearRaw[0], C.clearRaw[0]);
+                if (GEN && bytes == 2u) v.x = v.y = v.z = v.w = (v.x & 0xffffu) * 0x10001u;
+                if (GEN && bytes >= 8u) { v.y = v.w = C.clearRaw[1]; }
+                if (GEN && bytes == 16u) { v.z = C.clearRaw[2]; v.w = C.clearRaw[3]; }
                 for (uint32_t py = cy; py < min(cy + PF_TILE, C.H); py++) {
                     const size_t row = (size_t)py * C.W;
-                    if (!GEN && xe == cx + 8u && ((row + cx) & 3u) == 0 && !(C.clearMode == 1 && row + cx < 8) &&
-                        (((uintptr_t)C.color | (uintptr_t)C.depth) & 15u) == 0) {
-                        const uint32_t cr = C.clearRaw[0];
+                    unsigned char *const at = (unsigned char *)C.color + (row + cx) * bytes;
+                    if (wide && xe == cx + 8u && ((row + cx) & 3u) == 0 && !(C.clearMode == 1 && row + cx < 8) &&
+                        (((uintptr_t)at | (uintptr_t)C.depth) & 15u) == 0) {
                         const float cd = C.clearDepth;
-                        uint4 *cp = reinterpret_cast<uint4 *>((uint32_t *)C.color + row + cx);
+                        uint4 *cp = reinterpret_cast<uint4 *>(at);
                         float4 *dp = reinterpret_cast<float4 *>(C.depth + row + cx);
-                        cp[0] = make_uint4(cr, cr, cr, cr); cp[1] = make_uint4(cr, cr, cr, cr);
+                        for (uint32_t k = 0; k < bytes / 2u; k++) cp[k] = v;
                         dp[0] = make_float4(cd, cd, cd, cd); dp[1] = make_float4(cd, cd, cd, cd);
                         continue;
                     }
