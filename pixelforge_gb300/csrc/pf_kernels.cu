@@ -1864,12 +1864,10 @@ __device__ __forceinline__ uint32_t queue_refill(QWarp &Q, const uint32_t *bin, 
     uint32_t queued = left;
     bool lowering = Q.lowering != 0;
     const float farDepth = __int_as_float((int32_t)((farKey & 0x80000000u) ? farKey ^ 0x80000000u : ~farKey));
-    // No bound below 3e38: a record without one has none either.  NaN, which
-    // hides nothing, where the reciprocal of the farthest depth does not tell
-    // on which side of zero that is: for zeros and for infinities, before
-    // which every depth lies, negative ones too.
-    const float inv = !(fabsf(farDepth) < __int_as_float(0x7f800000)) ? __int_as_float(0x7fffffff) :
-                      farDepth > 0.0f ? fminf(__frcp_rn(farDepth) * 0.99999f, 3e38f) :
+    // No bound below 3e38: a record without one has none either; NaN, which
+    // hides nothing, for a zero.  (Before an infinity lies every depth, and
+    // its reciprocal has no sign: that is compared by the depth itself.)
+    const float inv = farDepth > 0.0f ? fminf(__frcp_rn(farDepth) * 0.99999f, 3e38f) :
                       farDepth < 0.0f ? __frcp_rn(farDepth) * 1.00001f : __int_as_float(0x7fffffff);
     const float fx = (float)ox, fy = (float)oy;
     while (queued < QCHN && c0 < n) {
@@ -1882,7 +1880,7 @@ __device__ __forceinline__ uint32_t queue_refill(QWarp &Q, const uint32_t *bin, 
         }
         lowering = __all_sync(0xffffffffu, p.w == p.w) && lowering;
         const float top = fminf(((p.x + p.y * fx) + p.z * fy) + (fmaxf(p.y * 7.0f, 0.0f) + fmaxf(p.z * 7.0f, 0.0f)), p.w);
-        const bool behind = lowering && top <= inv && (p.w > 0.0f) == (inv > 0.0f) && (key & ((1u << PF_SUB_BITS) - 1u)) == 0;
+        const bool behind = lowering && top <= inv && (p.w > 0.0f) == (farDepth > 0.0f) && (key & ((1u << PF_SUB_BITS) - 1u)) == 0;
         const uint32_t m = __ballot_sync(0xffffffffu, i < n && !behind);
         if ((m >> lane) & 1u) Q.keys[queued + __popc(m & ((1u << lane) - 1u))] = key;
         queued += __popc(m);
@@ -2173,17 +2171,20 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                 // (covered and visible already)
             } else if (kind == 0) {
                 // the whole box when no edge function is negative at its
-                // least corner (values in [-2^30, 2^30) and steps in
-                // [-2^24, 2^24): none wraps inside the tile; compared as
-                // unsigned, since -2^31 has no absolute value)
+                // least corner; values in [-2^30, 2^30) and steps in
+                // [-2^26, 2^26), of which none wraps inside the tile (-2^31,
+                // which has no absolute value, is outside as well)
                 bool full = bw + bh >= 12u;
-                if (full)
+                if (full) {
+                    uint32_t sign = 0, steps = 0;
 #pragma unroll
-                for (int e = 0; e < 3; e++) {
-                    const int32_t ex = e == 0 ? E.ex0 : e == 1 ? E.ex1 : E.ex2, ey = e == 0 ? E.ey0 : e == 1 ? E.ey1 : E.ey2;
-                    full = full && (uint32_t)E.e0[e] + (1u << 30) < (1u << 31) && (uint32_t)ex + (1u << 24) < (1u << 25) &&
-                           (uint32_t)ey + (1u << 24) < (1u << 25) &&
-                           E.e0[e] + (int32_t)(ex > 0 ? bx0 : bx0 + bw - 1u) * ex + (int32_t)(ey > 0 ? by0 : by0 + bh - 1u) * ey >= 0;
+                    for (int e = 0; e < 3; e++) {
+                        const uint32_t e0 = (uint32_t)E.e0[e], ex = (uint32_t)(e == 0 ? E.ex0 : e == 1 ? E.ex1 : E.ex2);
+                        const uint32_t ey = (uint32_t)(e == 0 ? E.ey0 : e == 1 ? E.ey1 : E.ey2);
+                        sign |= (e0 + (1u << 30)) | (e0 + ((int32_t)ex > 0 ? bx0 : bx0 + bw - 1u) * ex + ((int32_t)ey > 0 ? by0 : by0 + bh - 1u) * ey);
+                        steps |= (ex + (1u << 26)) | (ey + (1u << 26));
+                    }
+                    full = (sign >> 31 | steps >> 27) == 0;
                 }
                 const uint32_t cols = ((1u << bw) - 1u) << bx0;
                 if (full) {
