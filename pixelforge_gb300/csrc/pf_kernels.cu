@@ -1992,25 +1992,40 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
                 // (GEN: pixels of 2, 4, 8 or 16 bytes, the others pixel by pixel.
                 // Bound by the sectors L2 takes: a word a store, the sphere
                 // frame's raster sent it 14 M of RGBA float, most of them in part,
-                // and took 200 us with L2 full of written lines, 104 now; RGBA
-                // half 119 -> 105, 5-6-5 79 -> 71)
-                const uint32_t bytes = GEN ? (uint32_t)pff_bytes(C.fmt) : 4u;
-                const bool wide = !GEN || (bytes & (bytes - 1u)) == 0;
-                uint4 v = make_uint4(C.clearRaw[0], C.clearRaw[0], C.clearRaw[0], C.clearRaw[0]);
-                if (GEN && bytes == 2u) v.x = v.y = v.z = v.w = (v.x & 0xffffu) * 0x10001u;
-                if (GEN && bytes >= 8u) { v.y = v.w = C.clearRaw[1]; }
-                if (GEN && bytes == 16u) { v.z = C.clearRaw[2]; v.w = C.clearRaw[3]; }
+                // and took 200 us with L2 full of written lines, 100 now; RGBA
+                // half 119 -> 101, 5-6-5 79 -> 71.  Apart from the plain clear:
+                // one body for both cost that 0.5 % of the 64-soup batch)
+                uint4 v = make_uint4(0, 0, 0, 0);
+                uint32_t bytes = 0;
+                if (GEN) {
+                    const uint32_t b = (uint32_t)pff_bytes(C.fmt), c0 = C.clearRaw[0];
+                    if (b == 2u) { const uint32_t two = (c0 & 0xffffu) * 0x10001u; v = make_uint4(two, two, two, two); }
+                    else if (b == 4u) v = make_uint4(c0, c0, c0, c0);
+                    else if (b == 8u) v = make_uint4(c0, C.clearRaw[1], c0, C.clearRaw[1]);
+                    else v = make_uint4(c0, C.clearRaw[1], C.clearRaw[2], C.clearRaw[3]);
+                    bytes = (b & (b - 1u)) == 0 ? b : 0u;
+                }
                 for (uint32_t py = cy; py < min(cy + PF_TILE, C.H); py++) {
                     const size_t row = (size_t)py * C.W;
-                    unsigned char *const at = (unsigned char *)C.color + (row + cx) * bytes;
-                    if (wide && xe == cx + 8u && ((row + cx) & 3u) == 0 && !(C.clearMode == 1 && row + cx < 8) &&
-                        (((uintptr_t)at | (uintptr_t)C.depth) & 15u) == 0) {
+                    if (!GEN && xe == cx + 8u && ((row + cx) & 3u) == 0 && !(C.clearMode == 1 && row + cx < 8) &&
+                        (((uintptr_t)C.color | (uintptr_t)C.depth) & 15u) == 0) {
+                        const uint32_t cr = C.clearRaw[0];
                         const float cd = C.clearDepth;
-                        uint4 *cp = reinterpret_cast<uint4 *>(at);
+                        uint4 *cp = reinterpret_cast<uint4 *>((uint32_t *)C.color + row + cx);
                         float4 *dp = reinterpret_cast<float4 *>(C.depth + row + cx);
-                        for (uint32_t k = 0; k < bytes / 2u; k++) cp[k] = v;
+                        cp[0] = make_uint4(cr, cr, cr, cr); cp[1] = make_uint4(cr, cr, cr, cr);
                         dp[0] = make_float4(cd, cd, cd, cd); dp[1] = make_float4(cd, cd, cd, cd);
                         continue;
+                    }
+                    if (GEN && bytes && xe == cx + 8u && !(C.clearMode == 1 && row + cx < 8)) {
+                        uint4 *cp = reinterpret_cast<uint4 *>((unsigned char *)C.color + (row + cx) * bytes);
+                        float4 *dp = reinterpret_cast<float4 *>(C.depth + row + cx);
+                        if ((((uintptr_t)cp | (uintptr_t)dp) & 15u) == 0) {
+                            const float cd = C.clearDepth;
+                            for (uint32_t k = 0; k < bytes / 2u; k++) cp[k] = v;
+                            dp[0] = make_float4(cd, cd, cd, cd); dp[1] = make_float4(cd, cd, cd, cd);
+                            continue;
+                        }
                     }
                     for (uint32_t px = cx; px < xe; px++) {
                         const size_t pidx = row + px;
