@@ -635,8 +635,8 @@ __device__ __forceinline__ void list_tile(const BinArgs &B, uint32_t t, uint32_t
 // The same for the tiles of a whole warp (every lane calls it; lanes that
 // put nothing on a list pass added = 0): one atomic a list and warp.  The
 // five counters share a cache line, so an atomic per tile and level queues
-// there: the batch of 64 soups, 83,000 tiles past most levels, k_items 777
-// -> 645 us.
+// there: the batch of 64 soups, 83,000 tiles past most levels, 777 -> 645 us
+// of k_items in the first state of the binning below (312-326 now).
 __device__ __forceinline__ void list_tiles_warp(const BinArgs &B, uint32_t t, uint32_t before, uint32_t added)
 {
     const uint32_t from = heavy_level(before), to = heavy_level(before + added);
@@ -875,15 +875,15 @@ __device__ __noinline__ uint32_t clipped_pixels(const BinWarp &S, uint32_t recor
 // by the round trips of the counter atomics.  Testing every tile of the box
 // instead, one sub-triangle after the other, a batch of 64 soups (207,000
 // items covering hundreds of tiles each, 4.5 tiles tested per entry) took
-// 614 us, now 305; phong1080, whose triangles cover one or two tiles, 285
-// -> 217 us; the 2,000-triangle soup at 256x256 136 -> 17 us together with
-// the items a warp (pfd_launch_items).  Planes and fragment counts added
-// since cost 5 us of the batch and 40 of phong1080, and save k_raster 300
-// and 59 (queue_refill).  Pairs of one window of
-// 32 that touch the same tile share one atomic on its counter (neighbouring
-// triangles of a mesh usually do), slots within a group follow lane order;
-// the pairs of a single sub-triangle are distinct tiles and skip the
-// grouping.  The counters of BIN_BURST windows are claimed before any of
+// 614 us of k_items, now 312-326; phong1080, whose triangles cover one or two
+// tiles, 286 -> 229 us; the 2,000-triangle soup at 256x256 136 -> 17 us
+// together with the items a warp (pfd_launch_items).  Depth planes and
+// fragment counts are in the new figures: they cost 5 us of the batch and 40
+// of phong1080, and save k_raster 300 and 59 (queue_refill).  Pairs of one
+// window of 32 that touch the same tile share one atomic on its counter
+// (neighbouring triangles of a mesh usually do), slots within a group follow
+// lane order; the pairs of a single sub-triangle are distinct tiles and skip
+// the grouping.  The counters of BIN_BURST windows are claimed before any of
 // their slots is written, so that the atomics' round trips overlap.
 // Every lane of the warp must call it (lanes with nothing to bin pass
 // has = false).
@@ -1893,12 +1893,14 @@ __device__ __forceinline__ uint32_t queue_refill(QWarp &Q, const uint32_t *bin, 
 }
 
 // GEN: a target is not RGBA / unsigned byte.  PHONG: a draw state lights per
-// fragment; without that code nothing spills: sphere1080 58 -> 56 us,
-// 64-soup batch 1,925 -> 1,780.  Warps an SM, by what fits without spills:
-// 28 (72 registers; 24: 64-soup batch 1,555 -> 1,455, 8,192 small triangles
-// 32 -> 28; 32 warps: 1,505), GEN 24 (28: 35 -> 36.5 on RGBA half), PHONG 20
-// (24: phong1080 340 -> 312; 16: 362).  Bound by instruction issue and the
-// round trips of claims, bin keys and records.
+// fragment; launches without one do without that code: sphere1080 58 -> 56
+// us, 64-soup batch 1,925 -> 1,780.  Warps an SM, as measured: plain 28
+// (against 24: 64-soup batch 1,555 -> 1,455, 8,192 small triangles 32 -> 28;
+// 32 warps: 1,505), GEN 24 (28: 35 -> 36.5 on RGBA half), PHONG 20 (against
+// 24: phong1080 340 -> 312; 16: 362).  That leaves 72, 80 and 96 registers;
+// of the variants of 4 warps a CTA only the plain one does not spill (bytes
+// stored and loaded: GEN 8 and 16, PHONG 8 and 16, both 68 and 76).  Bound by
+// instruction issue and the round trips of claims, bin keys and records.
 template <bool GEN, int WARPS, bool PHONG>
 __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WARPS) k_raster(RasterArgs a)
 {
@@ -2412,8 +2414,14 @@ __global__ void __launch_bounds__(WARPS * 32, (PHONG ? 20 : GEN ? 24 : 28) / WAR
 // record by record, a lane a pixel.  Bound by that last chain: a record's
 // step reads its pixels, compares, blends and writes.  With one warp doing
 // all of it a record at a time (its load and its texels waited for in every
-// step) the sphere frame's launch at 1080p took 800 us; with a lane a half
-// in the drawing warp and one finding warp 240; this takes 177 us.
+// step) the sphere frame's launch at 1080p took 1,210 us, now 210, and 798
+// now 177 with the mesh turned, so that the small triangles around its poles
+// share no rows; with a lane a half in the drawing warp and one finding warp
+// 240 (turned).  Five CTAs an SM were chosen without per-fragment lighting
+// (six: 184), where 72 registers do.  With it they spill 136 bytes: a lit
+// frame (81,920 triangles, four lights, 1280x720) takes 1,113 us on the
+// device (3,002 before), and 1,060 with four CTAs, whose 96 registers do not
+// spill.
 // ---------------------------------------------------------------------------
 #define ROW_THREADS 160
 #define ROW_BATCH 32                // records of a batch
